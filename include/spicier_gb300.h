@@ -739,8 +739,9 @@ int sp_moments_device(sp_ctx* ctx, const double* d_values, uint64_t rows, uint32
 /* dispatch.rs:85-120).  A setting applies to the sizes of one bucket: key */
 /* "<setting>@<bucket>", bucket = sp_tune_bucket(size) (the smallest power */
 /* of two >= size, at least 4).  Settings and their size:                  */
-/*   lu.cta               1: CTA-per-system batched LU even where one      */
-/*                        thread per system fits (n <= 28); size n         */
+/*   lu.cta               1: CTA-per-system batched LU where the rule      */
+/*                        picks one thread per system (FP64 n <= 16,       */
+/*                        mixed n <= 28); size n                           */
 /*   newton.block.fp64 | .mixed | .exact  threads per block of the generic */
 /*                        thread-per-sample Newton kernels; size MNA n     */
 /*   spec.bpsm.fp64 | .mixed  resident blocks per SM of the topology-      */

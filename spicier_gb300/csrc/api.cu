@@ -278,14 +278,20 @@ static int solve_batch_device_locked(sp_ctx* ctx, const double* d_m, const doubl
     if (n > (size_t)kMaxBatchLuN)
         return fail(ctx, SP_ERR_INVALID_DIMENSION, "n = %zu exceeds the batched dense LU limit %d", n,
                     kMaxBatchLuN);
-    // one thread per system up to kMaxDenseN unknowns unless the tuner chose
-    // the CTA-per-system kernel for this size (setting "lu.cta", 1 = CTA)
-    const bool cta = n > (size_t)kMaxDenseN || tune_get(ctx, "lu.cta", (long long)n, 0) == 1;
+    // one thread per system for small systems, where a CTA's barriers and its
+    // per-column search cost more than the update (65,535 systems, thread / CTA:
+    // n = 14 0.58 / 0.97 ms, n = 16 0.97 / 1.18, n = 17 1.57 / 1.29, n = 28
+    // 11.5 / 3.4: a thread's n^2 doubles of shared memory leave one warp per SM
+    // there).  The mixed kernel, half the shared memory, keeps one thread per
+    // system up to kMaxDenseN; the tuner may choose the CTA kernel below either
+    // limit (setting "lu.cta", 1 = CTA).
+    const size_t thread_max = precision == SP_PREC_MIXED ? (size_t)kMaxDenseN : 16;
+    const bool cta = n > thread_max || tune_get(ctx, "lu.cta", (long long)n, 0) == 1;
     if (cta) {
         // one CTA per system, FP64 in the reference's order (both precisions)
         ProfScope prof(ctx, "lu_batch_cta", st);
         double* work = nullptr;
-        int grid = (int)std::min<size_t>(batch, (size_t)ctx->num_sms * 8);
+        int grid = (int)std::min<size_t>(batch, (size_t)ctx->num_sms * 32);
         if (lu_batch_cta_smem((int)n) > (size_t)ctx->max_smem - 1024) {
             const size_t per = lu_batch_cta_smem((int)n);
             grid = (int)std::max<size_t>(1, std::min<size_t>({batch, (size_t)ctx->num_sms * 2, ((size_t)4 << 30) / per}));

@@ -87,7 +87,7 @@ inline cudaError_t allow_dynamic_smem(const void* f, int max_smem) {
 struct AcLaunch;
 cudaError_t launch_ac(const AcLaunch& L, int grid, int block, size_t smem, cudaStream_t st);
 cudaError_t launch_ac_mixed(const AcLaunch& L, int grid, int block, size_t smem, cudaStream_t st);
-// solve_batch for n > kMaxDenseN: one CTA per system (shared memory when
+// solve_batch with one CTA per system (shared memory when
 // lu_batch_cta_smem(n) fits, else work = grid slices of n*n + n doubles)
 constexpr int kMaxBatchLuN = 4096;
 size_t lu_batch_cta_smem(int n);

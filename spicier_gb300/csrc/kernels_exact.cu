@@ -261,114 +261,155 @@ cudaError_t launch_lu_batch_exact(const double* mats, const double* rhs, int n, 
     return cudaGetLastError();
 }
 
-// The same solve for n beyond the one-thread-per-system limit: one CTA per
-// system.  Each step's pivot search (warp 0: first index of the largest
-// |a|, NaN never chosen, the diagonal kept when it is NaN), row swap,
-// scaling and rank-1 update touch every element in the order and with the
-// operations of lu_solve_fp64, only spread over threads, so the solution is
-// bit-identical.  A and b live in shared memory when they fit, else in a
+// a / b as IEEE division gives it, on the integer pipe wherever both operands
+// and the quotient are normal (a quotient of a zero is that zero with the
+// operands' sign), in hardware otherwise.
+__device__ __forceinline__ double lu_div(double a, double b) {
+    const uint64_t sign = (cr::dbits(a) ^ cr::dbits(b)) & (1ULL << 63);
+    const double q = ieee_div(fabs(a), fabs(b));
+    return cr::bdouble((cr::dbits(q) & ~(1ULL << 63)) | sign);
+}
+
+// The same solve with one CTA per system.  Each step's pivot search (warp 0:
+// first index of the largest |a|, NaN never chosen, the diagonal kept when it
+// is NaN), row swap, scaling and rank-1 update apply to every element the
+// operations of lu_solve_fp64 in the same order, only spread over threads, so
+// the solution is bit-identical.  The right-hand side is column n of A: the
+// update of that column is the forward substitution, so L needs no row swaps
+// and is not read again.  A lives in shared memory when it fits, else in a
 // per-CTA slice of global memory (work).
-__global__ void __launch_bounds__(256) lu_batch_cta_kernel(const double* __restrict__ mats,
+//
+// Bound: the FP64 pipe, two lanes per clock and SM, whatever the number of
+// active lanes; so nothing but the update's multiply and subtract runs on it.
+// The trailing block's elements are dealt to full warps in column-major order
+// (a warp that took rows of one column would idle on average a third of its
+// lanes), the pivot search compares bit patterns, and the divisions, one per
+// column and one per back-substitution step, run once per system on the
+// integer pipe.  Warp 0 updates column i + 1 first and searches it while the
+// other warps take the rest of the block in chunks.  65,535 systems of n = 50:
+// 13.9 ms, 1.5 times the pipe's time for the multiplies and subtracts (29.1 ms
+// with rows of a column per warp, the reciprocal in every warp and FP64
+// compares); 2,000 of n = 100: 3.5 ms (5.0).  The multiply on the integer pipe
+// beside the pipe's subtract measured slower (2.0 times at n = 50).
+constexpr int kLuChunk = 4;  // elements per lane of one chunk
+
+template <bool IN_WORK>
+__global__ void __launch_bounds__(512) lu_batch_cta_kernel(const double* __restrict__ mats,
                                                            const double* __restrict__ rhs, int n, uint64_t batch,
                                                            double* __restrict__ sol, uint8_t* __restrict__ sing,
                                                            double* __restrict__ work) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int s_piv[2];
-    __shared__ double s_diag[2];
-    __shared__ int s_bad;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+    __shared__ int s_piv, s_bad;
+    __shared__ double s_inv;
+    __shared__ int s_next[2];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const size_t nn = (size_t)n * n;
-    double* A = work ? work + (size_t)blockIdx.x * (nn + n) : reinterpret_cast<double*>(smem);
-    double* b = A + nn;
+    double* A = IN_WORK ? work + (size_t)blockIdx.x * (nn + n) : reinterpret_cast<double*>(smem);
+    // warp 0: pivot of column i into s_piv, 1 / pivot into s_inv, a zero pivot into s_bad
+    auto find_pivot = [&](int i) {
+        const double* col = A + (size_t)i * n;
+        const uint64_t inf = 0x7FF0000000000000ULL;
+        int piv = i;
+        if ((cr::dbits(col[i]) << 1) <= (inf << 1)) {
+            uint64_t best = 0;
+            int bi = i;
+            for (int r = i + lane; r < n; r += 32) {
+                const uint64_t v = cr::dbits(col[r]) & ~(1ULL << 63);
+                if (v > best && v <= inf) best = v, bi = r;
+            }
+            const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+            const bool top = (unsigned)(best >> 32) == hi;
+            const unsigned lo = __reduce_max_sync(0xffffffffu, top ? (unsigned)best : 0u);
+            piv = (int)__reduce_min_sync(0xffffffffu, top && (unsigned)best == lo ? (unsigned)bi : 0x7fffffffu);
+            // a column of zeros: every lane holds best = 0 and lane 0's index is i
+        }
+        const double diag = col[piv];
+        const bool zero = (cr::dbits(diag) << 1) == 0;
+        const double inv = zero ? 0.0 : lu_div(1.0, diag);
+        if (lane == 0) {
+            s_piv = piv;
+            s_inv = inv;
+            if (zero) s_bad = 1;
+        }
+    };
     for (uint64_t s = blockIdx.x; s < batch; s += gridDim.x) {
         const double* m = mats + s * nn;
         for (size_t k = tid; k < nn; k += blockDim.x) A[k] = m[k];
-        for (int k = tid; k < n; k += blockDim.x) b[k] = rhs[s * n + k];
+        for (int k = tid; k < n; k += blockDim.x) A[nn + k] = rhs[s * n + k];
+        if (tid == 0) s_bad = 0, s_next[0] = s_next[1] = 0;
         __syncthreads();
-        for (int i = 0; i < n; ++i) {
-            double* col = A + (size_t)i * n;  // column i: entries (r, i), r = 0..n-1
-            if (wid == 0) {
-                int piv = i;
-                if (!isnan(col[i])) {
-                    double best = -1.0;
-                    int bi = n;
-                    for (int r = i + lane; r < n; r += 32) {
-                        const double v = fabs(col[r]);
-                        if (v > best) {
-                            best = v;
-                            bi = r;
-                        }
-                    }
-#pragma unroll
-                    for (int o = 16; o; o >>= 1) {
-                        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                        if (ob > best || (ob == best && oi < bi)) {
-                            best = ob;
-                            bi = oi;
-                        }
-                    }
-                    piv = bi;
-                }
-                if (lane == 0) {
-                    s_piv[i & 1] = piv;
-                    s_diag[i & 1] = col[piv];
-                }
-            }
-            __syncthreads();
-            const int piv = s_piv[i & 1];
-            const double diag = s_diag[i & 1];
-            if (diag == 0.0) continue;
-            if (piv != i) {
-                for (int c = tid; c < n; c += blockDim.x) {
+        if (wid == 0) find_pivot(0);
+        __syncthreads();
+        for (int i = 0; i < n && !s_bad; ++i) {
+            // swap rows i and piv in columns i.. n, scale column i below the diagonal
+            const int piv = s_piv;
+            const double inv = s_inv;
+            double* col = A + (size_t)i * n;
+            if (piv != i)
+                for (int c = i + 1 + tid; c <= n; c += blockDim.x) {
                     double* cc = A + (size_t)c * n;
                     const double t = cc[i];
                     cc[i] = cc[piv];
                     cc[piv] = t;
                 }
-                if (tid == 0) {
-                    const double t = b[i];
-                    b[i] = b[piv];
-                    b[piv] = t;
-                }
-                __syncthreads();
-            }
-            const double inv = 1.0 / diag;
-            for (int r = i + 1 + tid; r < n; r += blockDim.x) col[r] = col[r] * inv;
+            const double cii = col[i], cpi = col[piv];
+            __syncthreads();  // every thread has read the column's two entries
+            for (int r = i + 1 + tid; r < n; r += blockDim.x) col[r] = (r == piv ? cii : col[r]) * inv;
+            if (tid == 0) col[i] = cpi, s_next[(i + 1) & 1] = 0;
             __syncthreads();
-            for (int c = i + 1 + wid; c < n; c += nw) {
-                double* cc = A + (size_t)c * n;
-                const double p = cc[i];
-                for (int r = i + 1 + lane; r < n; r += 32) cc[r] = -p * col[r] + cc[r];
+            const int rows = n - 1 - i;
+            if (rows == 0) break;
+            const double* l = col + i + 1;
+            if (wid == 0) {  // column i + 1, then its pivot
+                double* cc = A + (size_t)(i + 1) * n + i;
+                const double p = cc[0];
+                for (int r = lane; r < rows; r += 32) cc[1 + r] = -p * l[r] + cc[1 + r];
+                __syncwarp();
+                find_pivot(i + 1);
+            }
+            // columns i + 2 .. n, element e of the block at row e % rows, column e / rows
+            const int total = rows * rows;
+            const int q32 = 32 / rows, r32 = 32 - q32 * rows;
+            double* blk = A + (size_t)(i + 2) * n + i;
+            while (true) {
+                int e0 = 0;
+                if (lane == 0) e0 = atomicAdd(&s_next[i & 1], 32 * kLuChunk);
+                e0 = __shfl_sync(0xffffffffu, e0, 0);
+                if (e0 >= total) break;
+                int e = e0 + lane, c = e / rows, r = e - c * rows;
+                double a[kLuChunk], p[kLuChunk], f[kLuChunk];
+                int at[kLuChunk];  // the element's index in blk, -1 past the end
+#pragma unroll
+                for (int u = 0; u < kLuChunk; ++u) {
+                    const bool live = e + 32 * u < total;
+                    const int rr = live ? r : 0, k = (live ? c : 0) * n;
+                    at[u] = live ? k + 1 + rr : -1;
+                    a[u] = blk[k + 1 + rr];
+                    p[u] = blk[k];
+                    f[u] = l[rr];
+                    r += r32;
+                    c += q32;
+                    if (r >= rows) r -= rows, ++c;
+                }
+#pragma unroll
+                for (int u = 0; u < kLuChunk; ++u)
+                    if (at[u] >= 0) blk[at[u]] = -p[u] * f[u] + a[u];
             }
             __syncthreads();
         }
-        // substitutions by warp 0 (warp-synchronous)
-        if (wid == 0) {
-            for (int i = 0; i < n; ++i) {
-                const double coeff = b[i];
-                const double* col = A + (size_t)i * n;
-                for (int r = i + 1 + lane; r < n; r += 32) b[r] = -coeff * col[r] + b[r];
-                __syncwarp();
-            }
-            bool ok = true;
+        const bool bad = s_bad != 0;
+        double* b = A + nn;
+        if (wid == 0 && !bad) {  // back substitution (warp-synchronous); the diagonal is nonzero
             for (int i = n - 1; i >= 0; --i) {
                 const double* col = A + (size_t)i * n;
-                const double diag = col[i];
-                if (diag == 0.0) {
-                    ok = false;
-                    break;
-                }
-                const double coeff = b[i] / diag;
+                const double coeff = lu_div(b[i], col[i]);
                 __syncwarp();
                 if (lane == 0) b[i] = coeff;
                 for (int r = lane; r < i; r += 32) b[r] = -coeff * col[r] + b[r];
                 __syncwarp();
             }
-            if (lane == 0) s_bad = ok ? 0 : 1;
         }
         __syncthreads();
-        const bool bad = s_bad != 0;
         for (int k = tid; k < n; k += blockDim.x) sol[s * n + k] = bad ? 0.0 : b[k];
         if (tid == 0) sing[s] = bad ? 1 : 0;
         __syncthreads();  // before the next system overwrites A and b
@@ -381,7 +422,16 @@ cudaError_t launch_lu_batch_cta(const double* mats, const double* rhs, int n, ui
                                 uint8_t* sing, double* work, int grid, cudaStream_t st) {
     if (batch == 0) return cudaSuccess;
     const size_t smem = work ? 0 : lu_batch_cta_smem(n);
-    lu_batch_cta_kernel<<<grid, 256, smem, st>>>(mats, rhs, n, batch, sol, sing, work);
+    // threads per system: enough to spread a step's (n - i)^2 elements, few
+    // enough that its two barriers stay cheap.  Measured, ms for one batch per
+    // n at 32 / 64 / 128 / 256 / 512 threads: n = 20 (65,535 systems) 1.70 /
+    // 1.88 / 2.5 / - / -; n = 50 (16,500) 4.9 / 4.2 / 3.5 / 4.5 / -; n = 72
+    // (5,858) 7.1 / 4.5 / 4.1 / 3.6 / -; n = 100 (2,500) - / 8.8 / 5.6 / 4.9 / 4.4
+    const int block = n <= 22 ? 32 : n <= 40 ? 64 : n <= 64 ? 128 : n <= 88 ? 256 : 512;
+    if (work)
+        lu_batch_cta_kernel<true><<<grid, block, 0, st>>>(mats, rhs, n, batch, sol, sing, work);
+    else
+        lu_batch_cta_kernel<false><<<grid, block, smem, st>>>(mats, rhs, n, batch, sol, sing, work);
     return cudaGetLastError();
 }
 
@@ -410,7 +460,7 @@ cudaError_t prepare_exact_kernels(int max_smem) {
                          (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_FP64>,
                          (const void*)SP_KERNEL_NS::transient_fixed_kernel,
                          (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT>, (const void*)ac_kernel,
-                         (const void*)lu_batch_fp64_kernel, (const void*)lu_batch_cta_kernel};
+                         (const void*)lu_batch_fp64_kernel, (const void*)lu_batch_cta_kernel<false>};
     for (const void* f : fns) {
         cudaError_t e = allow_dynamic_smem(f, max_smem);
         if (e != cudaSuccess) return e;
