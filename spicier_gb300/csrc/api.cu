@@ -1007,7 +1007,8 @@ static int ladder_validate(sp_ctx* ctx, const sp_ladder_config* c, uint64_t coun
 }
 
 struct LadderPlan {
-    int stride;
+    bool ws;  // the per-section arrays in the global workspace (too long for shared memory)
+    int threads;
     size_t smem;
     uint64_t blocks;
     size_t bh, bo, bn, bw;
@@ -1016,22 +1017,21 @@ struct LadderPlan {
 
 static LadderPlan ladder_plan(const sp_ctx* ctx, const sp_ladder_config* c, uint64_t count) {
     LadderPlan p;
-    p.stride = (c->max_sections + 2 + 31) & ~31;
-    // four warps x (diag, rhs, c', d', block unknowns): FP64 elements, or FP32 in
-    // the mixed mode, whose smaller footprint leaves the SM's L1 to the
-    // per-ladder arrays
-    p.smem = (size_t)4 * ladder_warp_doubles(p.stride, c->precision) * 8;
-    // resident blocks per SM: the kernel's launch bounds allow two (registers), shared memory may allow fewer
-    int bpsm = std::max(1, std::min(2, (int)((228 * 1024 - 1024) / (p.smem + 1024))));
+    p.smem = ladder_smem(c->max_sections, c->precision, false);
+    p.ws = p.smem > (size_t)ctx->max_smem;
+    if (p.ws) p.smem = ladder_smem(c->max_sections, c->precision, true);
+    p.threads = ladder_threads(c->max_sections);
+    // resident blocks per SM by shared memory and by registers (the launch bounds allow 128 a thread)
+    int bpsm = std::max(1, std::min((int)(228 * 1024 / (p.smem + 1024)), 65536 / (128 * p.threads)));
     // tuned resident blocks per SM (setting "ladder.bpsm"), never above what fits
     const int tb = tune_get(const_cast<sp_ctx*>(ctx), "ladder.bpsm", c->max_sections, 0);
     if (tb >= 1 && tb < bpsm) bpsm = tb;
-    p.blocks = std::min<uint64_t>((count + 3) / 4, (uint64_t)ctx->num_sms * bpsm);
+    p.blocks = std::min<uint64_t>(count, (uint64_t)ctx->num_sms * bpsm);
     const int bins = c->max_sections - c->min_sections + 1;
     p.bh = align256(4 * (size_t)bins);
     p.bo = align256(4 * count);
     p.bn = 256;
-    p.bw = align256((size_t)p.blocks * 4 * LA_COUNT * p.stride * 8);
+    p.bw = p.ws ? align256((size_t)p.blocks * LA_COUNT * ((size_t)c->max_sections + 2) * 8) : 0;
     return p;
 }
 
@@ -1040,10 +1040,9 @@ static int ladder_locked(sp_ctx* ctx, const sp_ladder_config* c, uint64_t seed, 
                          double* d_probe, size_t extra, cudaStream_t st, double* d_steps = nullptr,
                          int max_rec = 0) {
     const LadderPlan p = ladder_plan(ctx, c, count);
-    if (p.smem > (size_t)ctx->max_smem) return fail(ctx, SP_ERR_INVALID_DIMENSION, "ladder too long for shared memory");
-    const int stride = p.stride;
-    const size_t smem = p.smem, bh = p.bh, bo = p.bo, bn = p.bn;
-    const uint64_t blocks = p.blocks;
+    if (p.smem > (size_t)ctx->max_smem || c->max_sections > ladder_max_sections(c->precision))
+        return fail(ctx, SP_ERR_INVALID_DIMENSION, "ladder too long for shared memory");
+    const size_t bh = p.bh, bo = p.bo, bn = p.bn;
     int rc = ensure_scratch(ctx, extra + p.bytes());
     if (rc) return rc;
     char* b = (char*)ctx->scratch + extra;
@@ -1055,9 +1054,7 @@ static int ladder_locked(sp_ctx* ctx, const sp_ladder_config* c, uint64_t seed, 
     unsigned int* hist = (unsigned int*)b;
     L.order = (const uint32_t*)(b + bh);
     L.next = (unsigned int*)(b + bh + bo);
-    L.ws = (double*)(b + bh + bo + bn);
-    L.stride = stride;
-    L.slots = (int)(blocks * 4);
+    L.ws = p.ws ? (double*)(b + bh + bo + bn) : nullptr;
     L.x_final = d_x;
     L.n = d_n;
     L.accepted = d_acc;
@@ -1071,9 +1068,9 @@ static int ladder_locked(sp_ctx* ctx, const sp_ladder_config* c, uint64_t seed, 
     static const char* names[3] = {"ladder_transient_fp64", "ladder_transient_mixed", "ladder_transient_fp64_exact"};
     ProfScope prof(ctx, names[c->precision], st);
     if (c->precision == SP_PREC_FP64_EXACT)
-        SP_CUDA(ctx, launch_ladder_exact(L, (int)blocks, smem, st), "ladder launch");
+        SP_CUDA(ctx, launch_ladder_exact(L, (int)p.blocks, p.threads, p.smem, st), "ladder launch");
     else
-        SP_CUDA(ctx, launch_ladder_fast(L, c->precision, (int)blocks, smem, st), "ladder launch");
+        SP_CUDA(ctx, launch_ladder_fast(L, c->precision, (int)p.blocks, p.threads, p.smem, st), "ladder launch");
     return SP_OK;
 }
 

@@ -61,9 +61,10 @@ cudaError_t launch_transient_fast(const TransientLaunch& L, int block, size_t sm
 struct LadderLaunch;
 struct GridLaunch;
 cudaError_t launch_grid(const GridLaunch& L, int precision, cudaStream_t st);
-// Ladder transient launchers (ladder.cuh): 128-thread blocks, one warp per instance.
-cudaError_t launch_ladder_exact(const LadderLaunch& L, int grid, size_t smem, cudaStream_t st);
-cudaError_t launch_ladder_fast(const LadderLaunch& L, int precision, int grid, size_t smem, cudaStream_t st);
+// Ladder transient launchers (ladder.cuh): one block of `threads` per instance.
+cudaError_t launch_ladder_exact(const LadderLaunch& L, int grid, int threads, size_t smem, cudaStream_t st);
+cudaError_t launch_ladder_fast(const LadderLaunch& L, int precision, int grid, int threads, size_t smem,
+                               cudaStream_t st);
 cudaError_t launch_ladder_prelude(const sp_ladder_config& c, uint64_t seed, uint64_t first, uint64_t count,
                                   unsigned int* hist, uint32_t* order, unsigned int* next, cudaStream_t st);
 

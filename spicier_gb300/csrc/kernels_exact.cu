@@ -444,8 +444,11 @@ cudaError_t launch_ac(const AcLaunch& L, int grid, int block, size_t smem, cudaS
     return cudaGetLastError();
 }
 
-cudaError_t launch_ladder_exact(const LadderLaunch& L, int grid, size_t smem, cudaStream_t st) {
-    SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT><<<grid, 128, smem, st>>>(L);
+cudaError_t launch_ladder_exact(const LadderLaunch& L, int grid, int threads, size_t smem, cudaStream_t st) {
+    if (L.ws)
+        SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT, true><<<grid, threads, smem, st>>>(L);
+    else
+        SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT, false><<<grid, threads, smem, st>>>(L);
     return cudaGetLastError();
 }
 
@@ -459,7 +462,8 @@ cudaError_t prepare_exact_kernels(int max_smem) {
     const void* fns[] = {(const void*)SP_KERNEL_NS::newton_primary_kernel<SP_PREC_FP64>,
                          (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_FP64>,
                          (const void*)SP_KERNEL_NS::transient_fixed_kernel,
-                         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT>, (const void*)ac_kernel,
+                         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT, false>,
+                         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT, true>, (const void*)ac_kernel,
                          (const void*)lu_batch_fp64_kernel, (const void*)lu_batch_cta_kernel<false>};
     for (const void* f : fns) {
         cudaError_t e = allow_dynamic_smem(f, max_smem);

@@ -486,11 +486,18 @@ cudaError_t launch_ladder_prelude(const sp_ladder_config& c, uint64_t seed, uint
     return cudaGetLastError();
 }
 
-cudaError_t launch_ladder_fast(const LadderLaunch& L, int precision, int grid, size_t smem, cudaStream_t st) {
-    if (precision == SP_PREC_MIXED)
-        SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED><<<grid, 128, smem, st>>>(L);
+cudaError_t launch_ladder_fast(const LadderLaunch& L, int precision, int grid, int threads, size_t smem,
+                               cudaStream_t st) {
+    using namespace SP_KERNEL_NS;
+    const bool ws = L.ws != nullptr;
+    if (precision == SP_PREC_MIXED && ws)
+        ladder_kernel<SP_PREC_MIXED, true><<<grid, threads, smem, st>>>(L);
+    else if (precision == SP_PREC_MIXED)
+        ladder_kernel<SP_PREC_MIXED, false><<<grid, threads, smem, st>>>(L);
+    else if (ws)
+        ladder_kernel<SP_PREC_FP64, true><<<grid, threads, smem, st>>>(L);
     else
-        SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64><<<grid, 128, smem, st>>>(L);
+        ladder_kernel<SP_PREC_FP64, false><<<grid, threads, smem, st>>>(L);
     return cudaGetLastError();
 }
 
@@ -574,7 +581,8 @@ cudaError_t prepare_fast_kernels(int max_smem) {
     const void* fns[] = {
         (const void*)SP_KERNEL_NS::grid_kernel<SP_PREC_MIXED>, (const void*)SP_KERNEL_NS::grid_kernel<SP_PREC_FP64>,
         (const void*)SP_KERNEL_NS::transient_fixed_kernel, (const void*)ac_mixed_kernel,
-        (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED>, (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64>,
+        (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED, false>, (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED, true>,
+        (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64, false>, (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64, true>,
         (const void*)SP_KERNEL_NS::newton_primary_kernel<SP_PREC_MIXED>, (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_MIXED>,
         (const void*)SP_KERNEL_NS::newton_primary_kernel<SP_PREC_FP64>, (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_FP64>,
         (const void*)lu_batch_mixed_kernel, (const void*)lu_batch_escalate_kernel};
