@@ -429,7 +429,18 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     for (int k = 0; k < c->num_params; ++k)
         if (c->params[k].kind != SP_DRAW_FIXED) drawn.push_back(k);
     size_t bw = align256(sizeof(int) * drawn.size());
-    cudaError_t e = cudaMalloc(&t->dev, be + bp + bu + bo + bn + bw + 256);
+    // the elements a fixed-step transient's right-hand side reads
+    std::vector<TransientEl> tran;
+    for (int pass = 0; pass < 3; ++pass)
+        for (int e = 0; e < c->num_elements; ++e) {
+            const sp_element& el = c->elements[e];
+            const bool src = el.kind == SP_EL_V || el.kind == SP_EL_I;
+            if (pass == 0 ? !src : el.kind != (pass == 1 ? SP_EL_C : SP_EL_L)) continue;
+            tran.push_back(TransientEl{el.node[0], el.node[1],
+                                       !src ? el.field[0] : (el.wave >= 0 ? el.wave : -1 - el.field[0]), el.kind});
+        }
+    const size_t bt = align256(sizeof(TransientEl) * tran.size());
+    cudaError_t e = cudaMalloc(&t->dev, be + bp + bu + bo + bn + bw + bt + 256);
     if (e != cudaSuccess) {
         delete t;
         return cuda_fail(ctx, e, "topology allocation");
@@ -441,7 +452,9 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     int* ddoff = (int*)(b + be + bp + bu);
     double* dns = (double*)(b + be + bp + bu + bo);
     int* ddrawn = (int*)(b + be + bp + bu + bo + bn);
-    if (c->num_elements) e = cudaMemcpy(del, c->elements, sizeof(sp_element) * c->num_elements, cudaMemcpyHostToDevice);
+    TransientEl* dtran = (TransientEl*)(b + be + bp + bu + bo + bn + bw);
+    if (!tran.empty()) e = cudaMemcpy(dtran, tran.data(), sizeof(TransientEl) * tran.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && c->num_elements) e = cudaMemcpy(del, c->elements, sizeof(sp_element) * c->num_elements, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !drawn.empty())
         e = cudaMemcpy(ddrawn, drawn.data(), sizeof(int) * drawn.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && c->num_params)
@@ -458,6 +471,7 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     }
     t->dc = DevCircuit{c->num_nodes, c->num_branches, t->n, c->num_elements, c->num_params, nd,
                        del, dpar, dpul, ddoff, c->nodeset ? dns : nullptr};
+    t->d_tran = dtran;
     t->d_drawn = ddrawn;
     t->num_drawn = (int)drawn.size();
     t->h_elements.assign(c->elements, c->elements + c->num_elements);
@@ -1308,22 +1322,33 @@ static int transient_locked(sp_ctx* ctx, sp_topology* t, const sp_newton_config*
                             const sp_transient_config* tc, uint64_t seed, uint64_t first, uint64_t count,
                             const double* d_table, uint32_t cols, double* d_x, double* d_probe, uint8_t* d_status,
                             cudaStream_t st) {
-    int nv = 0, ncap = 0, nind = 0;
+    int nv = 0, nsrc = 0, ncap = 0, nind = 0;
     for (const sp_element& el : t->h_elements) {
         const int k = el.kind;
         if (k != SP_EL_R && k != SP_EL_C && k != SP_EL_L && k != SP_EL_V && k != SP_EL_I)
             return fail(ctx, SP_ERR_INVALID_ARGUMENT, "fixed-step transients take linear circuits (R, C, L, V, I), as "
                                                       "solve_transient");
         nv += k == SP_EL_V;
+        nsrc += k == SP_EL_V || k == SP_EL_I;
         ncap += k == SP_EL_C;
         nind += k == SP_EL_L;
     }
     const int nt = t->num_nodes + nv;
     const long steps = (long)std::ceil(tc->tstop / tc->tstep);
-    const size_t words = transient_words(nt, ncap, nind);
+    const int npul = t->num_pulses;
+    // waveforms are tabulated 32 steps at a time, fewer with many pulses (a 4 KB table per warp), none beyond 512
+    const int wave_steps = std::min(32, 512 / std::max(npul, 1));
+    bool keep = true;
+    auto bytes = [&](int block) {
+        return 8 * (transient_words(nt, ncap + nind, tc->method, keep) * block +
+                    transient_warp_words(nt, npul, wave_steps, tc->method) * ((block + 31) / 32));
+    };
+    if (bytes(1) > (size_t)ctx->max_smem) keep = false;  // hundreds of parallel C or L: recompute their conductances
     int block = 128;
-    while (block > 1 && words * 8 * block > 110 * 1024) block >>= 1;
-    if (words * 8 * block > (size_t)ctx->max_smem) return fail(ctx, SP_ERR_INVALID_DIMENSION, "circuit too large");
+    while (block > 1 && bytes(block) > 110 * 1024) block >>= 1;
+    if (bytes(block) > (size_t)ctx->max_smem) return fail(ctx, SP_ERR_INVALID_DIMENSION, "circuit too large");
+    // a small sweep runs as one-warp blocks, so that it covers every SM
+    while (block > 32 && count / block < 2 * (uint64_t)ctx->num_sms) block >>= 1;
     const int ndc = t->n, np = t->num_params;
     const size_t bx = align256(8 * (size_t)ndc * count), bp = align256(8 * (size_t)std::max(np, 1) * count);
     int rc = ensure_aux(ctx, bx + bp);
@@ -1346,14 +1371,19 @@ static int transient_locked(sp_ctx* ctx, sp_topology* t, const sp_newton_config*
     L.tstop = tc->tstop;
     L.steps = steps;
     L.nt = nt;
+    L.els = (const TransientEl*)t->d_tran;
+    L.num_src = nsrc;
     L.num_caps = ncap;
     L.num_inds = nind;
+    L.num_pulses = npul;
+    L.keep = keep;
+    L.wave_steps = wave_steps;
     L.probe_idx = tc->probe;
     L.x = d_x;
     L.probe = d_probe;
     L.status = d_status;
     ProfScope prof(ctx, tc->precision == SP_PREC_FP64_EXACT ? "transient_fixed_exact" : "transient_fixed_fp64", st);
-    const size_t smem = words * 8 * block;
+    const size_t smem = bytes(block);
     if (tc->precision == SP_PREC_FP64_EXACT) SP_CUDA(ctx, launch_transient_exact(L, block, smem, st), "transient launch");
     else SP_CUDA(ctx, launch_transient_fast(L, block, smem, st), "transient launch");
     return SP_OK;

@@ -266,6 +266,7 @@ struct sp_topology {
     uint32_t min_table_cols = 0;  // 1 + largest table column any parameter reads
     void* dev = nullptr;  // one allocation: elements, params, pulses, doff, nodeset, drawn slots
     sp::DevCircuit dc{};
+    void* d_tran = nullptr;  // TransientEl[]: sources, capacitors, inductors, each in element order (inside `dev`)
     int* d_drawn = nullptr;  // slots whose kind is not SP_DRAW_FIXED, ascending (inside `dev`)
     int num_drawn = 0;
     // host copy of the description (for the specialiser)

@@ -1,6 +1,7 @@
 // Kernels that reproduce the reference's IEEE operation sequence.
 // Compiled with --fmad=false: no a*b+c is fused, as in the Rust reference.
 #define SP_KERNEL_NS kexact
+#define SP_EXACT_UNIT
 #include "internal.h"
 #include <math_constants.h>
 

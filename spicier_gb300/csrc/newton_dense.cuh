@@ -69,11 +69,10 @@ struct ResidSink {
     __device__ void rhs_set(int r, double v) { F[r] -= v; }
 };
 
-// nalgebra-order partial-pivot LU solve of A (column-major, A[c*n+r]) with
-// b overwritten by x.  The row permutation is applied to b as it is found,
-// which is the order in which LU::solve replays it.  Returns false on a zero
-// pivot (the system is singular).
-__device__ inline bool lu_solve_fp64(int n, Il<double> A, Il<double> b) {
+// nalgebra-order partial-pivot LU of A in place (column-major, A[c*n+r]); the
+// row permutation is applied to b as it is found, which is the order in which
+// LU::solve replays it.  A zero on the diagonal afterwards: singular.
+__device__ inline void lu_factor_fp64(int n, Il<double> A, Il<double> b) {
     for (int i = 0; i < n; ++i) {
         int piv = i;
         double best = fabs(A[i * n + i]);
@@ -103,6 +102,12 @@ __device__ inline bool lu_solve_fp64(int n, Il<double> A, Il<double> b) {
             for (int r = i + 1; r < n; ++r) A[c * n + r] = -p * A[i * n + r] + A[c * n + r];
         }
     }
+}
+
+// The solve: factorisation, then b overwritten by x.  Returns false on a zero
+// pivot (the system is singular).
+__device__ inline bool lu_solve_fp64(int n, Il<double> A, Il<double> b) {
+    lu_factor_fp64(n, A, b);
     for (int i = 0; i < n; ++i) {
         double coeff = b[i];
         for (int r = i + 1; r < n; ++r) b[r] = -coeff * A[i * n + r] + b[r];
