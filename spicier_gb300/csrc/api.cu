@@ -46,13 +46,19 @@ int ensure_scratch(sp_ctx* ctx, size_t bytes) {
     return ::grow_buffer(ctx, &ctx->scratch, &ctx->scratch_bytes, bytes, "scratch");
 }
 
-// Threads per block of the thread-per-sample kernels: the largest multiple of
-// 32 up to 128 whose shared-memory work area stays within ~110 KB (two blocks
-// per SM on a 228 KB SM).
-int pick_block(size_t per_thread, int max_smem) {
-    int block = 128;
-    while (block > 32 && per_thread * block > 110 * 1024) block -= 32;
-    if (per_thread * block > (size_t)max_smem) return 0;
+// Threads per block of the thread-per-sample kernels: the multiple of 32 up to
+// 128 that leaves the most warps resident by shared memory (the larger one of
+// equals; the op-amp's 1,344 bytes a thread: five one-warp blocks per SM, four
+// warps at 64), and one warp where the sweep would not cover every SM.
+int pick_block(size_t per_thread, int max_smem, uint64_t count, int num_sms) {
+    int block = 0, most = 0;
+    for (int b = 128; b >= 32; b -= 32) {
+        const size_t bytes = per_thread * b;
+        if (bytes > (size_t)max_smem) continue;
+        const int warps = std::min<int>((int)(228 * 1024 / (bytes + 1024)), 2048 / b) * (b / 32);
+        if (warps > most) block = b, most = warps;
+    }
+    while (block > 32 && count / block < (uint64_t)num_sms) block -= 32;
     return block;
 }
 
@@ -677,7 +683,7 @@ static int newton_dc_locked(sp_ctx* ctx, const sp_topology* t, const sp_newton_c
     const int kprec = prec == SP_PREC_MIXED ? SP_PREC_MIXED : SP_PREC_FP64;
     size_t per = kprec == SP_PREC_MIXED ? work_bytes_per_thread<SP_PREC_MIXED>(t->n)
                                         : work_bytes_per_thread<SP_PREC_FP64>(t->n);
-    int block = pick_block(per, ctx->max_smem);
+    int block = pick_block(per, ctx->max_smem, count, ctx->num_sms);
     if (!block) return fail(ctx, SP_ERR_INVALID_DIMENSION, "MNA size %d does not fit shared memory", t->n);
     {
         // tuned threads per block (setting "newton.block.<precision>"), within what shared memory allows

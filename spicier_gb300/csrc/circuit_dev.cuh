@@ -15,6 +15,8 @@
 #pragma once
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "../../include/spicier_gb300.h"
 #include "cr_math.cuh"
 
@@ -80,18 +82,35 @@ __host__ __device__ inline double limit_voltage(double vd, double nvt, double vc
     return vd;
 }
 
+#if defined(__CUDACC__)
+// a < b for finite a, b from their bit patterns (the integer pipe); -0 counts as below +0
+__device__ __forceinline__ bool below_int(double a, double b) {
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return (x ^ (long long)((unsigned long long)(x >> 63) >> 1)) < (y ^ (long long)((unsigned long long)(y >> 63) >> 1));
+}
+#endif
+
 // Level-1 evaluate (level1.rs:154-191); vth = |VTO|, beta = KP*NF*W/L.
+// INT_TESTS: the region tests as integer comparisons, for finite voltages (a
+// comparison is an FP64-pipe instruction; a zero's sign does not change the result).
+template <bool INT_TESTS = false>
 __host__ __device__ inline void mos_eval(bool pmos, double vth, double beta, double lambda, double vgs,
                                 double vds, double& ids, double& gds, double& gm) {
     if (pmos) {
         vgs = -vgs;
         vds = -vds;
     }
-    if (vgs < vth) {
+    auto below = [](double a, double b) {
+#if defined(__CUDA_ARCH__)
+        if (INT_TESTS) return below_int(a, b);
+#endif
+        return a < b;
+    };
+    if (below(vgs, vth)) {
         ids = 0.0;
         gds = 1e-12;
         gm = 0.0;
-    } else if (vds < vgs - vth) {
+    } else if (below(vds, vgs - vth)) {
         double vov = vgs - vth;
         double i = beta * (vov * vds - 0.5 * vds * vds) * (1.0 + lambda * vds);
         double g = beta * (vov - vds) * (1.0 + lambda * vds) +
@@ -413,6 +432,37 @@ struct SoA {
 // Mode of a stamping pass (Netlist::stamp_nonlinear_into, _scaled, + gmin).
 enum StampMode { STAMP_PLAIN = 0, STAMP_GMIN = 1, STAMP_SCALED = 2 };
 
+// Sinks that declare kIntTests take finite voltages only (see mos_eval).
+template <class S, class = void>
+struct sink_int_tests {
+    static constexpr bool value = false;
+};
+template <class S>
+struct sink_int_tests<S, typename std::enable_if<S::kIntTests>::type> {
+    static constexpr bool value = true;
+};
+
+// Stamps of a Level-1 MOSFET, in the reference's order; a sink may bring its own.
+template <class Sink>
+__host__ __device__ inline void stamp_mos(Sink& k, int d, int g, int so, double gds, double gm, double ieq) {
+    if (d >= 0) k.add(d, d, gds);
+    if (so >= 0) k.add(so, so, gds);
+    if (d >= 0 && so >= 0) {
+        k.add(d, so, -gds);
+        k.add(so, d, -gds);
+    }
+    if (d >= 0) {
+        if (g >= 0) k.add(d, g, gm);
+        if (so >= 0) k.add(d, so, -gm);
+    }
+    if (so >= 0) {
+        if (g >= 0) k.add(so, g, -gm);
+        k.add(so, so, gm);
+    }
+    if (d >= 0) k.rhs_add(d, -ieq);
+    if (so >= 0) k.rhs_add(so, ieq);
+}
+
 // Stamp every element linearised at the sink's current x.
 // Sink API: double x(int i); void add(int r, int c, double v);
 //           void rhs_add(int r, double v); void rhs_set(int r, double v).
@@ -490,25 +540,9 @@ __host__ __device__ inline void stamp_all(const DevCircuit& c, const SoA& dv, si
                 double vs = so >= 0 ? k.x(so) : 0.0;
                 double vgs = vg - vs, vds = vd - vs;
                 double ids, gds, gm;
-                mos_eval(el.kind == SP_EL_PMOS, dv(off, s), dv(off + 1, s), dv(off + 2, s), vgs, vds,
-                         ids, gds, gm);
-                if (d >= 0) k.add(d, d, gds);
-                if (so >= 0) k.add(so, so, gds);
-                if (d >= 0 && so >= 0) {
-                    k.add(d, so, -gds);
-                    k.add(so, d, -gds);
-                }
-                if (d >= 0) {
-                    if (g >= 0) k.add(d, g, gm);
-                    if (so >= 0) k.add(d, so, -gm);
-                }
-                if (so >= 0) {
-                    if (g >= 0) k.add(so, g, -gm);
-                    k.add(so, so, gm);
-                }
-                double ieq = ids - gds * vds - gm * vgs;
-                if (d >= 0) k.rhs_add(d, -ieq);
-                if (so >= 0) k.rhs_add(so, ieq);
+                mos_eval<sink_int_tests<Sink>::value>(el.kind == SP_EL_PMOS, dv(off, s), dv(off + 1, s), dv(off + 2, s),
+                                                      vgs, vds, ids, gds, gm);
+                stamp_mos(k, d, g, so, gds, gm, ids - gds * vds - gm * vgs);
                 break;
             }
             case SP_EL_NPN:

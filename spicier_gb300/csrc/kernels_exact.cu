@@ -262,15 +262,6 @@ cudaError_t launch_lu_batch_exact(const double* mats, const double* rhs, int n, 
     return cudaGetLastError();
 }
 
-// a / b as IEEE division gives it, on the integer pipe wherever both operands
-// and the quotient are normal (a quotient of a zero is that zero with the
-// operands' sign), in hardware otherwise.
-__device__ __forceinline__ double lu_div(double a, double b) {
-    const uint64_t sign = (cr::dbits(a) ^ cr::dbits(b)) & (1ULL << 63);
-    const double q = ieee_div(fabs(a), fabs(b));
-    return cr::bdouble((cr::dbits(q) & ~(1ULL << 63)) | sign);
-}
-
 // The same solve with one CTA per system.  Each step's pivot search (warp 0:
 // first index of the largest |a|, NaN never chosen, the diagonal kept when it
 // is NaN), row swap, scaling and rank-1 update apply to every element the
@@ -326,7 +317,7 @@ __global__ void __launch_bounds__(512) lu_batch_cta_kernel(const double* __restr
         }
         const double diag = col[piv];
         const bool zero = (cr::dbits(diag) << 1) == 0;
-        const double inv = zero ? 0.0 : lu_div(1.0, diag);
+        const double inv = zero ? 0.0 : div_int(1.0, diag);
         if (lane == 0) {
             s_piv = piv;
             s_inv = inv;
@@ -403,7 +394,7 @@ __global__ void __launch_bounds__(512) lu_batch_cta_kernel(const double* __restr
         if (wid == 0 && !bad) {  // back substitution (warp-synchronous); the diagonal is nonzero
             for (int i = n - 1; i >= 0; --i) {
                 const double* col = A + (size_t)i * n;
-                const double coeff = lu_div(b[i], col[i]);
+                const double coeff = div_int(b[i], col[i]);
                 __syncwarp();
                 if (lane == 0) b[i] = coeff;
                 for (int r = lane; r < i; r += 32) b[r] = -coeff * col[r] + b[r];
