@@ -446,7 +446,18 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
                                        !src ? el.field[0] : (el.wave >= 0 ? el.wave : -1 - el.field[0]), el.kind});
         }
     const size_t bt = align256(sizeof(TransientEl) * tran.size());
-    cudaError_t e = cudaMalloc(&t->dev, be + bp + bu + bo + bn + bw + bt + 256);
+    // Gaussian slots' mean and sigma as FP32 pairs; a NaN sigma (never decided in
+    // FP32) where either is far from 1, so that no error term underflows
+    std::vector<float4> gauss(c->num_params);
+    for (int k = 0; k < c->num_params; ++k) {
+        const sp_param& q = c->params[k];
+        const double m = std::fabs(q.a), sg = std::fabs(q.b);
+        const bool fine = q.kind == SP_DRAW_GAUSS && (m == 0.0 || (m >= 0x1p-60 && m <= 0x1p60)) && sg >= 0x1p-60 && sg <= 0x1p60;
+        const float mh = (float)q.a, sh = (float)q.b;
+        gauss[k] = fine ? make_float4(mh, (float)(q.a - mh), sh, (float)(q.b - sh)) : make_float4(0.f, 0.f, NAN, 0.f);
+    }
+    const size_t bg = align256(sizeof(float4) * gauss.size());
+    cudaError_t e = cudaMalloc(&t->dev, be + bp + bu + bo + bn + bw + bt + bg + 256);
     if (e != cudaSuccess) {
         delete t;
         return cuda_fail(ctx, e, "topology allocation");
@@ -459,7 +470,9 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     double* dns = (double*)(b + be + bp + bu + bo);
     int* ddrawn = (int*)(b + be + bp + bu + bo + bn);
     TransientEl* dtran = (TransientEl*)(b + be + bp + bu + bo + bn + bw);
-    if (!tran.empty()) e = cudaMemcpy(dtran, tran.data(), sizeof(TransientEl) * tran.size(), cudaMemcpyHostToDevice);
+    float4* dgauss = (float4*)(b + be + bp + bu + bo + bn + bw + bt);
+    if (!gauss.empty()) e = cudaMemcpy(dgauss, gauss.data(), sizeof(float4) * gauss.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !tran.empty()) e = cudaMemcpy(dtran, tran.data(), sizeof(TransientEl) * tran.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && c->num_elements) e = cudaMemcpy(del, c->elements, sizeof(sp_element) * c->num_elements, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !drawn.empty())
         e = cudaMemcpy(ddrawn, drawn.data(), sizeof(int) * drawn.size(), cudaMemcpyHostToDevice);
@@ -478,6 +491,7 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     t->dc = DevCircuit{c->num_nodes, c->num_branches, t->n, c->num_elements, c->num_params, nd,
                        del, dpar, dpul, ddoff, c->nodeset ? dns : nullptr};
     t->d_tran = dtran;
+    t->d_gauss32 = dgauss;
     t->d_drawn = ddrawn;
     t->num_drawn = (int)drawn.size();
     t->h_elements.assign(c->elements, c->elements + c->num_elements);
@@ -637,6 +651,19 @@ static int newton_dc_locked(sp_ctx* ctx, const sp_topology* t, const sp_newton_c
     if (!D.derive && !D.x0_out && !D.params_out &&
         (!warm || mlp_inputs_drawn(warm, t->h_params.data(), t->num_params)))
         D.next_items = reinterpret_cast<unsigned long long*>(s.counters + 6);
+    // the double-float kernel rounds every parameter to FP32, so a sweep in which
+    // nothing else reads the draws (no residual, returned parameters, network or
+    // linear term read from memory) draws FP32 values; the fallback draws the
+    // samples it takes over in FP64
+    const int* lin_slots = nullptr;
+    const float *lin_w = nullptr, *lin_io = nullptr;
+    const bool draw32 = pmode && !D.derive && !D.params_out && !d_resid &&
+                        (!warm || (linear_warm && mlp_linear_host(warm, &lin_w, &lin_io, &lin_slots) &&
+                                   spec_linear_as_parameter(t, prec, lin_slots, lin.lin_nin)));
+    if (draw32) {
+        D.params32 = (float*)s.params;
+        D.gauss32 = t->d_gauss32;
+    }
     {
         ProfScope prof(ctx, "draw_params", st);
         SP_CUDA(ctx, launch_draw(D, st), "draw launch");
@@ -675,6 +702,10 @@ static int newton_dc_locked(sp_ctx* ctx, const sp_topology* t, const sp_newton_c
         L.params = s.params;
         L.params_stride = count;
         L.derived_out = s.derived;
+        if (draw32) {
+            L.params32 = (const float*)s.params;
+            L.redraw = RedrawArgs{seed, first_index, d_table, table_cols, s.derived};
+        }
     }
     // with one sample per thread the specialised kernel reduces its blocks'
     // moments itself; a final kernel merges them (replacing the rows pass)

@@ -429,6 +429,15 @@ struct SoA {
     }
 };
 
+#if defined(__CUDACC__)
+// The same through L2, for a kernel that writes the arrays before it reads them.
+struct SoACg {
+    const double* p;
+    size_t stride;
+    __device__ double operator()(int slot, size_t s) const { return __ldcg(p + (size_t)slot * stride + s); }
+};
+#endif
+
 // Mode of a stamping pass (Netlist::stamp_nonlinear_into, _scaled, + gmin).
 enum StampMode { STAMP_PLAIN = 0, STAMP_GMIN = 1, STAMP_SCALED = 2 };
 
@@ -466,8 +475,8 @@ __host__ __device__ inline void stamp_mos(Sink& k, int d, int g, int so, double 
 // Stamp every element linearised at the sink's current x.
 // Sink API: double x(int i); void add(int r, int c, double v);
 //           void rhs_add(int r, double v); void rhs_set(int r, double v).
-template <class Sink>
-__host__ __device__ inline void stamp_all(const DevCircuit& c, const SoA& dv, size_t s, Sink& k, int mode,
+template <class DV, class Sink>
+__host__ __device__ inline void stamp_all(const DevCircuit& c, const DV& dv, size_t s, Sink& k, int mode,
                                  double aux) {
     const bool scaled = (mode == STAMP_SCALED);
     for (int e = 0; e < c.num_elements; ++e) {

@@ -39,6 +39,10 @@ struct DrawLaunch {
     const int* lin_slots = nullptr;
     int lin_nin = 0, lin_nout = 0;
     double* x0_out = nullptr;
+    // FP32 draws ([slot][count], drawn slots only) instead of params_soa, and the
+    // Gaussians' mean and sigma as FP32 pairs per slot (GaussF32)
+    float* params32 = nullptr;
+    const float4* gauss32 = nullptr;
     // false: skip the derived constants (the consumer, the double-float
     // specialised kernel, computes its constants from the parameters)
     bool derive = true;
@@ -266,6 +270,7 @@ struct sp_topology {
     uint32_t min_table_cols = 0;  // 1 + largest table column any parameter reads
     void* dev = nullptr;  // one allocation: elements, params, pulses, doff, nodeset, drawn slots
     sp::DevCircuit dc{};
+    const float4* d_gauss32 = nullptr;  // [num_params] mean and sigma of Gaussian slots as FP32 pairs (inside `dev`)
     void* d_tran = nullptr;  // TransientEl[]: sources, capacitors, inductors, each in element order (inside `dev`)
     int* d_drawn = nullptr;  // slots whose kind is not SP_DRAW_FIXED, ascending (inside `dev`)
     int num_drawn = 0;
@@ -289,6 +294,9 @@ int spec_prepare(sp_topology* t, int prec, std::string& err);
 bool spec_params_mode(const sp_topology* t, int prec);
 // True when the specialised kernel's grid gives every sample its own thread
 // (then it can reduce its blocks' moments itself).
+// True when the specialised kernel takes the linear warm start with these input
+// slots as a launch parameter (so that it reads no FP64 parameter).
+bool spec_linear_as_parameter(const sp_topology* t, int prec, const int* slots, int nin);
 bool spec_one_sample_per_thread(const sp_topology* t, int prec, uint64_t count);
 cudaError_t spec_launch(const sp_topology* t, int prec, const NewtonLaunch& L, cudaStream_t st);
 void spec_release_all(sp_ctx* ctx);

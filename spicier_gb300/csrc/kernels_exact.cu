@@ -13,21 +13,6 @@
 
 namespace sp {
 
-// Per-sample parameter draw (sp_draw_kind) and derived constants.
-// gaussian_scaled = mean + z * sigma (rng.rs:148-150), two roundings.
-__device__ inline double draw_one(const sp_param& p, uint64_t seed, uint32_t sweep,
-                                  const double* row, unsigned* hard) {
-    switch (p.kind) {
-        case SP_DRAW_FIXED: return p.a;
-        case SP_DRAW_GAUSS: return p.a + rng_gaussian(seed, sweep, p.rng_index, hard) * p.b;
-        case SP_DRAW_UNIFORM: return p.a + rng_uniform(seed, sweep, p.rng_index) * (p.b - p.a);
-        case SP_DRAW_LOGUNIFORM:
-            return p.a * cr_exp(rng_uniform(seed, sweep, p.rng_index) * cr_log(p.b / p.a, hard), hard);
-        case SP_DRAW_TABLE: return row ? row[p.rng_index] : CUDART_NAN;
-    }
-    return CUDART_NAN;
-}
-
 // Persistent draw kernel: each block takes groups of 32 samples from a
 // device counter (a static stride without one) and, per group,
 //
@@ -151,6 +136,38 @@ __global__ void __launch_bounds__(kDrawSamples * kDrawLanes, 4) draw_items_kerne
     if (hard && L.hard) atomicAdd(L.hard, hard);
 }
 
+// The draws of a sweep whose only consumer rounds them to FP32 (the
+// double-float Newton kernel): FP32 values, Gaussians without the full draw
+// where that decides the rounding (gauss_f32).  The work is even: a row of
+// blocks per drawn slot, whose warps take 32-sample groups by a fixed stride.
+__device__ __noinline__ static float draw_f32_full(const sp_param& p, uint64_t seed, uint32_t sweep, const double* row) {
+    return __double2float_rn(draw_one(p, seed, sweep, row, nullptr));
+}
+
+__global__ void __launch_bounds__(256, 4) draw_f32_kernel(DrawLaunch L) {
+    pdl_wait();
+    pdl_trigger();
+    const uint32_t lane = threadIdx.x & 31, groups = (uint32_t)((L.count + 31) / 32), warps = gridDim.x * 8;
+    for (int slot = blockIdx.y; slot < L.num_drawn; slot += gridDim.y) {
+        const int k = L.drawn[slot];
+        const sp_param p = L.c.par[k];
+        const uint64_t pk1 = (uint64_t)(p.rng_index * 2u) * 0x5851f42d4c957f2dULL;
+        const uint64_t pk2 = (uint64_t)(p.rng_index * 2u + 1u) * 0x5851f42d4c957f2dULL;
+        const float4 ms = L.gauss32[k];
+        float* out = L.params32 + (size_t)k * L.count;
+        for (uint32_t g = blockIdx.x * 8 + threadIdx.x / 32; g < groups; g += warps) {
+            const uint64_t s = (uint64_t)g * 32 + lane;
+            if (s >= L.count) continue;
+            const uint32_t sweep = (uint32_t)(L.first_index + s);
+            float v = 0.f;
+            bool done = false;
+            if (p.kind == SP_DRAW_GAUSS) done = gauss_f32(L.seed ^ (uint64_t)sweep * 0x517cc1b727220a95ULL, pk1, pk2, ms, &v);
+            if (!done) v = draw_f32_full(L.c.par[k], L.seed, sweep, L.table ? L.table + s * L.table_cols : nullptr);
+            out[s] = v;
+        }
+    }
+}
+
 cudaError_t launch_draw(const DrawLaunch& L, cudaStream_t st) {
     if (L.count == 0) return cudaSuccess;
     int dev = 0, sms = 0;
@@ -158,6 +175,15 @@ cudaError_t launch_draw(const DrawLaunch& L, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     const uint64_t groups = (L.count + kDrawSamples - 1) / kDrawSamples;
+    if (L.params32) {
+        if (L.num_drawn == 0) return cudaSuccess;
+        // one row of blocks per slot, about eight blocks per SM in all, and as few
+        // warps per row as take the same number of groups each
+        const uint64_t row = std::max<uint64_t>(1, ((uint64_t)sms * 8 + L.num_drawn - 1) / L.num_drawn);
+        const uint64_t each = (groups + row * 8 - 1) / (row * 8);
+        const uint64_t gx = (groups + each * 8 - 1) / (each * 8);
+        return launch_chained(draw_f32_kernel, dim3((unsigned)gx, (unsigned)std::min(L.num_drawn, 65535)), dim3(256), 0, st, L);
+    }
     if (L.next_items && !L.derive && !L.x0_out && !L.params_out) {
         if (L.num_drawn == 0) return cudaSuccess;
         const uint64_t warps = groups * (uint64_t)L.num_drawn;

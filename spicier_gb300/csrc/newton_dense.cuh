@@ -26,6 +26,7 @@
 //                   root of F, independent of the FP32 factorisation error.
 #pragma once
 #include "circuit_dev.cuh"
+#include "draw.cuh"
 #include "pdl.cuh"
 
 namespace sp {
@@ -405,8 +406,8 @@ __device__ inline bool step_ok(double old, double nw, double reltol, double abst
 }
 
 // One solve_newton_raphson from w.x; w.x holds the last iterate on return.
-template <int PREC>
-__device__ inline int newton_run(const DevCircuit& c, const SoA& dv, size_t s,
+template <int PREC, class DV>
+__device__ inline int newton_run(const DevCircuit& c, const DV& dv, size_t s,
                                  const sp_newton_config& cfg, int mode, double aux, Work& w,
                                  int& iters) {
     const int n = c.n;
@@ -520,7 +521,8 @@ __device__ inline int newton_run_warp(const DevCircuit& c, const SoA& dv, size_t
 }
 
 // max_i<num_nodes |F_i| of the FP64 KCL residual at w.x (uses w.v as scratch).
-__device__ inline double kcl_residual(const DevCircuit& c, const SoA& dv, size_t s, Work& w) {
+template <class DV>
+__device__ inline double kcl_residual(const DevCircuit& c, const DV& dv, size_t s, Work& w) {
     for (int i = 0; i < c.n; ++i) w.v[i] = 0.0;
     ResidSink k{w.v, w.x};
     stamp_all(c, dv, s, k, STAMP_PLAIN, 0.0);
@@ -564,6 +566,10 @@ struct NewtonLaunch {
     double* derived_out = nullptr;
     // per-block moments of the specialised kernel (one sample per thread), [n][grid]
     sp_moments* moments_partial = nullptr;
+    // FP32 drawn parameters of the specialised kernel ([slot][params_stride], then
+    // params is not read), and what the fallback needs to draw its samples in FP64
+    const float* params32 = nullptr;
+    RedrawArgs redraw;
     // iteration limit of the specialised kernel's cold restart of a sample
     // whose warm start missed (the full limit; cfg may hold the warm cap)
     int cold_max_iterations = 0;
@@ -647,8 +653,8 @@ __global__ void newton_primary_kernel(NewtonLaunch L) {
 // output row (global), the trial iterate in shared memory.  A failed attempt
 // is repeated by the reference with the identical initial guess and stamper,
 // so its outcome repeats; those repeats are accounted without recomputation.
-template <int PREC>
-__device__ inline int gmin_stepping(const NewtonLaunch& L, size_t s, Work& w, int& total) {
+template <int PREC, class DV>
+__device__ inline int gmin_stepping(const NewtonLaunch& L, const DV& dv, size_t s, Work& w, int& total) {
     const int n = L.c.n;
     const sp_newton_config& cfg = L.cfg;
     double* sol = L.x + s * n;
@@ -659,7 +665,7 @@ __device__ inline int gmin_stepping(const NewtonLaunch& L, size_t s, Work& w, in
         ++levels;
         for (int i = 0; i < n; ++i) w.x[i] = sol[i];
         int it = 0;
-        int code = newton_run<PREC>(L.c, L.dv, s, cfg, STAMP_GMIN, g, w, it);
+        int code = newton_run<PREC>(L.c, dv, s, cfg, STAMP_GMIN, g, w, it);
         total += it;
         if (code == NR_SINGULAR) return NR_SINGULAR;
         if (code != NR_CONVERGED) {
@@ -675,8 +681,8 @@ __device__ inline int gmin_stepping(const NewtonLaunch& L, size_t s, Work& w, in
 }
 
 // source stepping (newton.rs:261-356).
-template <int PREC>
-__device__ inline int source_stepping(const NewtonLaunch& L, size_t s, Work& w, int& total) {
+template <int PREC, class DV>
+__device__ inline int source_stepping(const NewtonLaunch& L, const DV& dv, size_t s, Work& w, int& total) {
     const int n = L.c.n;
     const sp_newton_config& cfg = L.cfg;
     double* sol = L.x + s * n;
@@ -689,7 +695,7 @@ __device__ inline int source_stepping(const NewtonLaunch& L, size_t s, Work& w, 
         double cur = fmin(factor, 1.0);
         for (int i = 0; i < n; ++i) w.x[i] = sol[i];
         int it = 0;
-        int code = newton_run<PREC>(L.c, L.dv, s, cfg, STAMP_SCALED, cur, w, it);
+        int code = newton_run<PREC>(L.c, dv, s, cfg, STAMP_SCALED, cur, w, it);
         total += it;
         if (code == NR_SINGULAR) return NR_SINGULAR;
         if (code != NR_CONVERGED) {
@@ -722,8 +728,10 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
     const int n = L.c.n;
     const bool warm = L.x0 != nullptr || L.lin != nullptr;  // listed samples started warm
     const unsigned int misses = *L.fail_count;
+    const SoACg dv{L.dv.p, L.dv.stride};
     for (unsigned int j = blockIdx.x * blockDim.x + threadIdx.x; j < misses; j += gridDim.x * blockDim.x) {
         const size_t s = L.fail_list[j];
+        if (L.redraw.derived) redraw_sample(L.c, L.redraw, L.dv.stride, s);
         int total = L.iters ? L.iters[s] : 0;
         uint8_t flags = warm ? SP_ST_FLAG_WARM : 0;
         // A stage succeeds only if it converged with a finite iterate (the
@@ -743,23 +751,23 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
             flags |= SP_ST_FLAG_COLD;
             load_start(L, s, w, false);
             int it = 0;
-            code = newton_run<PREC>(L.c, L.dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
+            code = newton_run<PREC>(L.c, dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
             total += it;
             for (int i = 0; i < n; ++i) L.x[s * n + i] = w.x[i];
         }
         if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_GMIN)) {
             flags |= SP_ST_FLAG_GMIN;
-            code = gmin_stepping<PREC>(L, s, w, total);
+            code = gmin_stepping<PREC>(L, dv, s, w, total);
         }
         if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_SOURCE)) {
             flags |= SP_ST_FLAG_SOURCE;
-            code = source_stepping<PREC>(L, s, w, total);
+            code = source_stepping<PREC>(L, dv, s, w, total);
         }
         for (int i = 0; i < n; ++i) w.x[i] = L.x[s * n + i];
         uint8_t st = finish_status(code, w, n) | flags;
         if (L.iters) L.iters[s] = total;
         if (L.status) L.status[s] = st;
-        if (L.resid) L.resid[s] = kcl_residual(L.c, L.dv, s, w);
+        if (L.resid) L.resid[s] = kcl_residual(L.c, dv, s, w);
     }
 }
 

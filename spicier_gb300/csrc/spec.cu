@@ -191,6 +191,7 @@ struct SpecArgs {
     double* dvo;
     spx_mom* mom;
     int cold_max_it;
+    const float* lp32;
 };
 __device__ __forceinline__ bool spx_fin(double v) {  // not Inf / NaN, on the integer pipe
     return ((unsigned int)(__double_as_longlong(v) >> 32) & 0x7ff00000u) != 0x7ff00000u;
@@ -762,9 +763,15 @@ std::string generate(const sp_topology* t, const Pattern& P, bool fp32_jac) {
         // FP32 constants: |VTO|, ((KP NF) W) / L and LAMBDA, 1 / R, source values
         // (at most a few FP32 roundings from the FP64 constants rounded to FP32)
         ld << "  {\n";
+        for (int slot : pslots) ld << "  float pf" << slot << ";\n";
+        ld << "  if (a.lp32) {\n";
         for (int slot : pslots)
-            ld << "  const double pd" << slot << " = __ldg(a.lp + (u64)" << slot << " * a.lpstride + s);\n";
-        for (int slot : pslots) ld << "  const float pf" << slot << " = __double2float_rn(pd" << slot << ");\n";
+            ld << "    pf" << slot << " = __ldg(a.lp32 + (u64)" << slot << " * a.lpstride + s);\n";
+        ld << "  } else {\n";
+        for (int slot : pslots)
+            ld << "    const double pd" << slot << " = __ldg(a.lp + (u64)" << slot << " * a.lpstride + s);\n";
+        for (int slot : pslots) ld << "    pf" << slot << " = __double2float_rn(pd" << slot << ");\n";
+        ld << "  }\n";
         for (int e = 0; e < t->num_elements; ++e) {
             const sp_element& el = t->h_elements[e];
             const int d0 = doff[e];
@@ -927,7 +934,7 @@ std::string generate(const sp_topology* t, const Pattern& P, bool fp32_jac) {
     if (dfm) {
         // parameters mode: the FP64 constants of a listed sample (for the generic
         // fallback) or of a residual, from the sample's parameters
-        o << "    if (spx_miss || a.resid) {\n";
+        o << "    if ((spx_miss && !a.lp32) || a.resid) {\n";
         for (int slot : pslots)
             o << "      const double pd" << slot << " = __ldg(a.lp + (u64)" << slot << " * a.lpstride + s);\n";
         emit_derive64(o, t, doff, pe, "      ");
@@ -935,8 +942,11 @@ std::string generate(const sp_topology* t, const Pattern& P, bool fp32_jac) {
     }
     o << "    if (spx_miss) {\n"
       << "      unsigned int k = atomicAdd(a.fail_count, 1u); a.fail_list[k] = (unsigned int)s;\n";
-    if (dfm)
+    if (dfm) {  // (the fallback draws the samples of an FP32 sweep itself)
+        o << "      if (!a.lp32) {\n";
         for (int k = 0; k < t->num_derived; ++k) o << "      a.dvo[" << k << " * st + s] = c" << k << ";\n";
+        o << "      }\n";
+    }
     o << "    } else if (a.resid) {\n"
       << "    double F[" << n << "];\n    #pragma unroll\n    for (int i = 0; i < " << n << "; ++i) F[i] = 0.0;\n";
     emit_elements(o, t, P, doff, false);
@@ -1027,6 +1037,7 @@ struct SpecArgsHost {
     double* dvo;  // parameters mode: FP64 derived constants of the samples put on the miss list
     sp_moments* mom;  // per-block moments [n][grid] (one sample per thread), or nullptr
     int cold_max_it;  // iteration limit of the cold restart of a warm-start miss (0: none)
+    const float* lp32;  // FP32 drawn parameters [slot][lpstride] (lp is then not read)
 };
 
 bool spec_params_mode(const sp_topology* t, int prec) { return prec == SP_PREC_MIXED && df_supported(t); }
@@ -1111,6 +1122,26 @@ int spec_prepare(sp_topology* t, int prec, std::string& err) {
     return SP_OK;
 }
 
+// Where each of the linear term's input slots lies in the kernel's parameter
+// order; false when an input is not there or they are not ascending.
+static bool linear_slots_at(const LinLayout& ll, const int* slots, int nin, std::vector<int>& at) {
+    const int ps = (int)ll.slots.size();
+    at.assign(nin, -1);
+    bool ok = ll.usable && nin > 0;
+    for (int j = 0; ok && j < nin; ++j) {
+        ok = j == 0 || slots[j] > slots[j - 1];
+        for (int k = 0; ok && k < ps; ++k)
+            if (ll.slots[k] == slots[j]) at[j] = k;
+        ok = ok && at[j] >= 0;
+    }
+    return ok;
+}
+
+bool spec_linear_as_parameter(const sp_topology* t, int prec, const int* slots, int nin) {
+    std::vector<int> at;
+    return linear_slots_at(lin_layout(t, prec == SP_PREC_MIXED && df_supported(t)), slots, nin, at);
+}
+
 cudaError_t spec_launch(const sp_topology* t, int prec, const NewtonLaunch& L, cudaStream_t st) {
     const int slot = prec == SP_PREC_MIXED ? 0 : 1;
     SpecArgsHost a{};
@@ -1138,6 +1169,8 @@ cudaError_t spec_launch(const sp_topology* t, int prec, const NewtonLaunch& L, c
     a.lpstride = L.params ? L.params_stride : L.lin_pstride;
     a.dvo = L.derived_out;
     a.mom = L.moments_partial;
+    a.lp32 = L.params32;
+    if (a.lp32 && (!spec_params_mode(t, prec) || a.resid)) return cudaErrorInvalidValue;
     if (spec_params_mode(t, prec) && (!a.lp || !a.dvo)) return cudaErrorInvalidValue;
     a.lw = L.lin;
     a.lio = L.lin_io;
@@ -1148,16 +1181,10 @@ cudaError_t spec_launch(const sp_topology* t, int prec, const NewtonLaunch& L, c
     // kernel reads the term from memory)
     const LinLayout ll = lin_layout(t, prec == SP_PREC_MIXED && df_supported(t));
     std::vector<unsigned long long> lkbuf((16 + 4 * (size_t)ll.nw + 7) / 8, 0ull);
-    if (ll.usable && L.lin && L.lin_host && L.lin_io_host && L.lin_slots_host) {
+    if (L.lin && L.lin_host && L.lin_io_host && L.lin_slots_host) {
         const int ps = (int)ll.slots.size(), n = t->n, nin = L.lin_nin;
-        std::vector<int> at(nin, -1);
-        bool ok = nin > 0;
-        for (int j = 0; ok && j < nin; ++j) {
-            ok = j == 0 || L.lin_slots_host[j] > L.lin_slots_host[j - 1];
-            for (int k = 0; ok && k < ps; ++k)
-                if (ll.slots[k] == L.lin_slots_host[j]) at[j] = k;
-            ok = ok && at[j] >= 0;
-        }
+        std::vector<int> at;
+        const bool ok = linear_slots_at(ll, L.lin_slots_host, nin, at);
         if (ok) {
             unsigned long long mask = 0;
             float* w = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(lkbuf.data()) + 16);
@@ -1171,6 +1198,7 @@ cudaError_t spec_launch(const sp_topology* t, int prec, const NewtonLaunch& L, c
             reinterpret_cast<int*>(lkbuf.data())[2] = 1;
         }
     }
+    if (a.lp32 && L.lin && !lkbuf[0]) return cudaErrorInvalidValue;  // that form reads FP64 parameters
     void* args[] = {&a, lkbuf.data()};
     // tuned resident blocks per SM (setting "spec.bpsm.<precision>"), never above the occupancy limit
     int bpsm = t->spec_bpsm[slot];
