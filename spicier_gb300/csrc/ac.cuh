@@ -22,6 +22,15 @@
 
 namespace sp {
 
+// A structurally nonzero real entry of the AC matrix; an element with
+// imaginary entries and the first of its values.
+struct AcEntry {
+    int16_t r, c;
+};
+struct AcReact {
+    int kind, n0, n1, n2, n3, val;
+};
+
 struct AcLaunch {
     DevCircuit c;
     const double* params;  // [count][np] the DC pass's drawn parameters
@@ -39,6 +48,15 @@ struct AcLaunch {
     double* work;           // global interleaved work area, or nullptr (shared memory)
     int refine;             // mixed kernel: FP64 residual refinement steps
     SoA dv;                 // the DC pass's per-sample derived constants (BSIM3 elements)
+    // FP64 sweeps (ac_sparse.cuh): the topology's lists, the samples' values and
+    // the samples that the dense kernel solves
+    const AcEntry* entries = nullptr;   // real entries of the matrix
+    const AcReact* reacts = nullptr;    // elements with imaginary entries
+    int num_entries = 0, num_reacts = 0, num_rvals = 0;
+    double* values = nullptr;           // [num_entries + num_rvals][count]
+    unsigned* redo = nullptr;           // [count]
+    unsigned* any_redo = nullptr;
+    int cap = 0;                        // value slots per thread
 };
 
 // BSIM3 small-signal values at the operating point x (ac_info_at,
@@ -193,29 +211,21 @@ __device__ inline bool ac_lu_solve(int n, CxArr A, CxArr b, int8_t* swap_with) {
     return true;
 }
 
-// One (sample, frequency) unit u = s * nf + f with the work area A.
-__device__ inline void ac_unit(const AcLaunch& L, uint64_t u, CxArr A) {
-    const uint64_t s = u / (uint64_t)L.nf;
-    const int f = (int)(u % (uint64_t)L.nf);
+// The frequency-independent part of a sample's system in the netlist stamper's
+// order: add(r, c, v) for every real entry (r or c may be -1), drive(row) for
+// every driven source.
+template <class AddF, class DriveF>
+__device__ inline void ac_real_stamps(const AcLaunch& L, uint64_t s, AddF add, DriveF drive) {
     const DevCircuit& c = L.c;
     const int n = c.n, nn = c.num_nodes;
-    double* out = L.out + (u * (uint64_t)L.num_probe) * 2;
-    if ((L.dc_status[s] & SP_ST_MASK) != SP_ST_CONVERGED) {
-        for (int k = 0; k < 2 * L.num_probe; ++k) out[k] = CUDART_NAN;
-        return;
-    }
-    const CxArr b{A.base + (int64_t)(2 * n * n) * A.stride, A.stride};
-    for (int k = 0; k < n * n; ++k) A[k].re() = 0.0, A[k].im() = 0.0;
-    for (int k = 0; k < n; ++k) b[k].re() = 0.0, b[k].im() = 0.0;
     const double* P = L.params + s * (uint64_t)L.np;
     const double* x = L.x_dc + s * (uint64_t)n;
     auto V = [&](int i) { return i >= 0 ? x[i] : 0.0; };
     auto cond = [&](int i, int j, double g) {
-        ac_add_re(A, n, i, i, g), ac_add_re(A, n, j, j, g), ac_add_re(A, n, i, j, -g), ac_add_re(A, n, j, i, -g);
+        add(i, i, g), add(j, j, g), add(i, j, -g), add(j, i, -g);
     };
     auto vccs = [&](int op, int on, int cp, int cn, double gm) {
-        ac_add_re(A, n, op, cp, gm), ac_add_re(A, n, op, cn, -gm), ac_add_re(A, n, on, cp, -gm),
-            ac_add_re(A, n, on, cn, gm);
+        add(op, cp, gm), add(op, cn, -gm), add(on, cp, -gm), add(on, cn, gm);
     };
     const double vt = thermal_voltage_300();
     for (int e = 0; e < c.num_elements; ++e) {
@@ -226,9 +236,9 @@ __device__ inline void ac_unit(const AcLaunch& L, uint64_t u, CxArr A) {
             case SP_EL_V:
             case SP_EL_L: {
                 const int br = nn + el.branch;
-                ac_add_re(A, n, a0, br, 1.0), ac_add_re(A, n, br, a0, 1.0);
-                ac_add_re(A, n, a1, br, -1.0), ac_add_re(A, n, br, a1, -1.0);
-                if (el.kind == SP_EL_V && (L.source < 0 || L.source == e)) b[br].re() += 1.0;
+                add(a0, br, 1.0), add(br, a0, 1.0);
+                add(a1, br, -1.0), add(br, a1, -1.0);
+                if (el.kind == SP_EL_V && (L.source < 0 || L.source == e)) drive(br);
                 break;
             }
             case SP_EL_D: {  // diode.rs evaluate at vd (it limits once)
@@ -273,6 +283,26 @@ __device__ inline void ac_unit(const AcLaunch& L, uint64_t u, CxArr A) {
                 break;
         }
     }
+}
+
+// One (sample, frequency) unit u = s * nf + f with the work area A.
+__device__ inline void ac_unit(const AcLaunch& L, uint64_t u, CxArr A) {
+    const uint64_t s = u / (uint64_t)L.nf;
+    const int f = (int)(u % (uint64_t)L.nf);
+    const DevCircuit& c = L.c;
+    const int n = c.n, nn = c.num_nodes;
+    double* out = L.out + (u * (uint64_t)L.num_probe) * 2;
+    if ((L.dc_status[s] & SP_ST_MASK) != SP_ST_CONVERGED) {
+        for (int k = 0; k < 2 * L.num_probe; ++k) out[k] = CUDART_NAN;
+        return;
+    }
+    const CxArr b{A.base + (int64_t)(2 * n * n) * A.stride, A.stride};
+    for (int k = 0; k < n * n; ++k) A[k].re() = 0.0, A[k].im() = 0.0;
+    for (int k = 0; k < n; ++k) b[k].re() = 0.0, b[k].im() = 0.0;
+    const double* P = L.params + s * (uint64_t)L.np;
+    const double* x = L.x_dc + s * (uint64_t)n;
+    ac_real_stamps(L, s, [&](int r, int cc, double v) { ac_add_re(A, n, r, cc, v); },
+                   [&](int br) { b[br].re() += 1.0; });
     const double wv = 2.0 * 3.141592653589793 * L.freqs[f];
     for (int e = 0; e < c.num_elements; ++e) {
         const sp_element el = c.el[e];
@@ -305,16 +335,19 @@ __device__ inline void ac_unit(const AcLaunch& L, uint64_t u, CxArr A) {
     }
 }
 
+// The dense solve of the samples the sparse kernel hands back (redo set).
 // Grid-stride over the units; thread t's work area is column t of the
 // interleaved shared (blockDim threads) or global (gridDim * blockDim) array.
 __global__ void __launch_bounds__(128) ac_kernel(AcLaunch L) {
+    if (*L.any_redo == 0) return;
     extern __shared__ __align__(16) unsigned char ac_smem[];
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
     const CxArr A = L.work ? CxArr{L.work + t, (int64_t)nthreads}
                            : CxArr{reinterpret_cast<double*>(ac_smem) + threadIdx.x, (int64_t)blockDim.x};
     const uint64_t total = L.count * (uint64_t)L.nf;
-    for (uint64_t u = t; u < total; u += nthreads) ac_unit(L, u, A);
+    for (uint64_t u = t; u < total; u += nthreads)
+        if (L.redo[u / (uint64_t)L.nf]) ac_unit(L, u, A);
 }
 
 __global__ void ac_status_kernel(uint64_t count, const uint8_t* dc_status, const unsigned int* singular,

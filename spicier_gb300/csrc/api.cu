@@ -11,6 +11,7 @@
 #include "ladder.cuh"
 #include "transient_fixed.cuh"
 #include "ac.cuh"
+#include "ac_sparse.cuh"
 #include "powergrid.cuh"
 
 using namespace sp;
@@ -457,7 +458,45 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
         gauss[k] = fine ? make_float4(mh, (float)(q.a - mh), sh, (float)(q.b - sh)) : make_float4(0.f, 0.f, NAN, 0.f);
     }
     const size_t bg = align256(sizeof(float4) * gauss.size());
-    cudaError_t e = cudaMalloc(&t->dev, be + bp + bu + bo + bn + bw + bt + bg + 256);
+    // the AC matrix's real entries (ac_real_stamps' positions, in order of first
+    // touch) and the elements with imaginary ones
+    std::vector<AcEntry> acent;
+    std::vector<AcReact> acreact;
+    int acvals = 0;
+    {
+        std::vector<char> seen((size_t)std::max(t->n, 1) * std::max(t->n, 1), 0);
+        auto put = [&](int r, int col) {
+            if (r < 0 || col < 0 || seen[(size_t)col * t->n + r]) return;
+            seen[(size_t)col * t->n + r] = 1;
+            acent.push_back(AcEntry{(int16_t)r, (int16_t)col});
+        };
+        auto cond = [&](int i, int j) { put(i, i), put(j, j), put(i, j), put(j, i); };
+        auto vccs = [&](int op, int on, int cp, int cn) { put(op, cp), put(op, cn), put(on, cp), put(on, cn); };
+        for (int e = 0; e < c->num_elements && t->n <= 256; ++e) {
+            const sp_element& el = c->elements[e];
+            const int a0 = el.node[0], a1 = el.node[1], a2 = el.node[2], a3 = el.node[3], br = c->num_nodes + el.branch;
+            switch (el.kind) {
+                case SP_EL_R:
+                case SP_EL_D: cond(a0, a1); break;
+                case SP_EL_V:
+                case SP_EL_L: put(a0, br), put(br, a0), put(a1, br), put(br, a1); break;
+                case SP_EL_NMOS:
+                case SP_EL_PMOS: cond(a0, a2), vccs(a0, a2, a1, a2); break;
+                case SP_EL_NPN:
+                case SP_EL_PNP: cond(a1, a2), cond(a0, a2), vccs(a0, a2, a1, a2); break;
+                case SP_EL_BSIM3N:
+                case SP_EL_BSIM3P: cond(a0, a2), vccs(a0, a2, a1, a2), vccs(a0, a2, a3, a2); break;
+                default: break;
+            }
+            const bool b3 = el.kind == SP_EL_BSIM3N || el.kind == SP_EL_BSIM3P;
+            if (el.kind != SP_EL_C && el.kind != SP_EL_L && !b3) continue;
+            acreact.push_back(AcReact{el.kind, el.kind == SP_EL_L ? br : a0, a1, a2, a3, acvals});
+            acvals += b3 ? 5 : 1;
+        }
+        for (AcReact& r : acreact) r.val += (int)acent.size();
+    }
+    const size_t bae = align256(sizeof(AcEntry) * acent.size()), bar = align256(sizeof(AcReact) * acreact.size());
+    cudaError_t e = cudaMalloc(&t->dev, be + bp + bu + bo + bn + bw + bt + bg + bae + bar + 256);
     if (e != cudaSuccess) {
         delete t;
         return cuda_fail(ctx, e, "topology allocation");
@@ -471,7 +510,11 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     int* ddrawn = (int*)(b + be + bp + bu + bo + bn);
     TransientEl* dtran = (TransientEl*)(b + be + bp + bu + bo + bn + bw);
     float4* dgauss = (float4*)(b + be + bp + bu + bo + bn + bw + bt);
-    if (!gauss.empty()) e = cudaMemcpy(dgauss, gauss.data(), sizeof(float4) * gauss.size(), cudaMemcpyHostToDevice);
+    char* dac = b + be + bp + bu + bo + bn + bw + bt + bg;
+    if (!acent.empty()) e = cudaMemcpy(dac, acent.data(), sizeof(AcEntry) * acent.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !acreact.empty())
+        e = cudaMemcpy(dac + bae, acreact.data(), sizeof(AcReact) * acreact.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !gauss.empty()) e = cudaMemcpy(dgauss, gauss.data(), sizeof(float4) * gauss.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !tran.empty()) e = cudaMemcpy(dtran, tran.data(), sizeof(TransientEl) * tran.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && c->num_elements) e = cudaMemcpy(del, c->elements, sizeof(sp_element) * c->num_elements, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && !drawn.empty())
@@ -492,6 +535,11 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
                        del, dpar, dpul, ddoff, c->nodeset ? dns : nullptr};
     t->d_tran = dtran;
     t->d_gauss32 = dgauss;
+    t->d_ac = dac;
+    t->ac_react_off = bae;
+    t->num_ac_entries = (int)acent.size();
+    t->num_ac_reacts = (int)acreact.size();
+    t->num_ac_values = acvals;
     t->d_drawn = ddrawn;
     t->num_drawn = (int)drawn.size();
     t->h_elements.assign(c->elements, c->elements + c->num_elements);
@@ -1556,8 +1604,11 @@ static int ac_locked(sp_ctx* ctx, sp_topology* t, const sp_newton_config* dc_cfg
     grid = std::max(grid, 1);
     const size_t bx = align256(8 * (size_t)n * count), bp = align256(8 * (size_t)np * count),
                  bf = align256(8 * (size_t)nf), bs = align256(4 * count),
-                 bw = shared ? 0 : align256(per * (size_t)grid * block);
-    int rc = ensure_aux(ctx, bx + bp + bf + bs + bw);
+                 bw = shared ? 0 : align256(per * (size_t)grid * block),
+                 // FP64: the samples' values, redo flags and their "any" word
+                 bv = mixed ? 0 : align256(8 * (size_t)(t->num_ac_entries + t->num_ac_values) * count),
+                 br = mixed ? 0 : align256(4 * count + 4);
+    int rc = ensure_aux(ctx, bx + bp + bf + bs + bw + bv + br);
     if (rc) return rc;
     char* base = (char*)ctx->aux;
     double* x_dc = (double*)base;
@@ -1566,7 +1617,9 @@ static int ac_locked(sp_ctx* ctx, sp_topology* t, const sp_newton_config* dc_cfg
     unsigned int* singular = (unsigned int*)(base + bx + bp + bf);
     double* work = shared ? nullptr : (double*)(base + bx + bp + bf + bs);
     SP_CUDA(ctx, cudaMemcpyAsync(d_freqs, freqs.data(), 8 * (size_t)nf, cudaMemcpyHostToDevice, st), "H2D freqs");
+    unsigned int* redo = (unsigned int*)(base + bx + bp + bf + bs + bw + bv);
     SP_CUDA(ctx, cudaMemsetAsync(singular, 0, 4 * count, st), "clear flags");
+    if (!mixed) SP_CUDA(ctx, cudaMemsetAsync(redo, 0, 4 * count + 4, st), "clear flags");
     rc = newton_dc_locked(ctx, t, dc_cfg, seed, first, count, d_table, cols, nullptr, x_dc, nullptr, d_status,
                           nullptr, params, nullptr, st);
     if (rc) return rc;
@@ -1594,7 +1647,33 @@ static int ac_locked(sp_ctx* ctx, sp_topology* t, const sp_newton_config* dc_cfg
     }
     ProfScope prof(ctx, mixed ? "ac_sweep_mixed" : "ac_sweep_fp64", st);
     if (mixed) SP_CUDA(ctx, launch_ac_mixed(L, grid, block, shared ? per * block : 0, st), "AC launch");
-    else SP_CUDA(ctx, launch_ac(L, grid, block, shared ? per * block : 0, st), "AC launch");
+    else {
+        L.entries = (const AcEntry*)t->d_ac;
+        L.reacts = (const AcReact*)((const char*)t->d_ac + t->ac_react_off);
+        L.num_entries = t->num_ac_entries;
+        L.num_reacts = t->num_ac_reacts;
+        L.num_rvals = t->num_ac_values;
+        L.values = (double*)(base + bx + bp + bf + bs + bw);
+        L.redo = redo;
+        L.any_redo = redo + count;
+        // slots per thread: the structural parts with as many again for fill, the
+        // right-hand side and the pivots' reciprocals; at most every part there is.
+        // A system that needs more is solved by the dense kernel.
+        const int all = 2 * n * (n + 1) + n;
+        L.cap = std::min(all, 2 * (t->num_ac_entries + 4 * t->num_ac_reacts) + 4 * n);
+        while (L.cap > 1 && ac_sparse_warp_bytes(n, L.cap) > (size_t)ctx->max_smem) --L.cap;
+        // the block that leaves the most warps resident
+        int sblock = 32, most = 0;
+        for (int w = 1; w <= 4; ++w) {
+            const size_t bytes = ac_sparse_warp_bytes(n, L.cap) * w;
+            if (bytes > (size_t)ctx->max_smem) break;
+            const int warps = std::min<int>((int)(228 * 1024 / (bytes + 1024)), 32) * w;
+            if (warps > most) sblock = 32 * w, most = warps;
+        }
+        const uint64_t groups = (units + sblock - 1) / sblock;
+        const int sgrid = (int)std::min<uint64_t>(groups, (uint64_t)ctx->num_sms * std::max(1, most / (sblock / 32)));
+        SP_CUDA(ctx, launch_ac(L, grid, block, shared ? per * block : 0, sgrid, sblock, st), "AC launch");
+    }
     return SP_OK;
 }
 

@@ -90,7 +90,8 @@ inline cudaError_t allow_dynamic_smem(const void* f, int max_smem) {
     return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem - (int)a.sharedSizeBytes);
 }
 struct AcLaunch;
-cudaError_t launch_ac(const AcLaunch& L, int grid, int block, size_t smem, cudaStream_t st);
+cudaError_t launch_ac(const AcLaunch& L, int grid, int block, size_t smem, int sparse_grid, int sparse_block,
+                      cudaStream_t st);
 cudaError_t launch_ac_mixed(const AcLaunch& L, int grid, int block, size_t smem, cudaStream_t st);
 // solve_batch with one CTA per system (shared memory when
 // lu_batch_cta_smem(n) fits, else work = grid slices of n*n + n doubles)
@@ -270,6 +271,9 @@ struct sp_topology {
     uint32_t min_table_cols = 0;  // 1 + largest table column any parameter reads
     void* dev = nullptr;  // one allocation: elements, params, pulses, doff, nodeset, drawn slots
     sp::DevCircuit dc{};
+    const void* d_ac = nullptr;  // AcEntry[num_ac_entries], then AcReact[num_ac_reacts] (inside `dev`)
+    size_t ac_react_off = 0;     // bytes
+    int num_ac_entries = 0, num_ac_reacts = 0, num_ac_values = 0;
     const float4* d_gauss32 = nullptr;  // [num_params] mean and sigma of Gaussian slots as FP32 pairs (inside `dev`)
     void* d_tran = nullptr;  // TransientEl[]: sources, capacitors, inductors, each in element order (inside `dev`)
     int* d_drawn = nullptr;  // slots whose kind is not SP_DRAW_FIXED, ascending (inside `dev`)

@@ -10,6 +10,7 @@
 #include "transient_fixed.cuh"
 #define SP_AC_KERNELS
 #include "ac.cuh"
+#include "ac_sparse.cuh"
 
 namespace sp {
 
@@ -453,7 +454,13 @@ cudaError_t launch_lu_batch_cta(const double* mats, const double* rhs, int n, ui
     return cudaGetLastError();
 }
 
-cudaError_t launch_ac(const AcLaunch& L, int grid, int block, size_t smem, cudaStream_t st) {
+cudaError_t launch_ac(const AcLaunch& L, int grid, int block, size_t smem, int sparse_grid, int sparse_block,
+                      cudaStream_t st) {
+    int vblock = 128;  // n^2 doubles of shared memory per sample
+    const size_t per = 8 * (size_t)L.c.n * L.c.n;
+    while (vblock > 32 && (per * vblock > 110 * 1024 || L.count / vblock < 304)) vblock >>= 1;
+    ac_values_kernel<<<(unsigned)((L.count + vblock - 1) / vblock), vblock, per * vblock, st>>>(L);
+    ac_sparse_kernel<<<sparse_grid, sparse_block, ac_sparse_warp_bytes(L.c.n, L.cap) * (sparse_block / 32), st>>>(L);
     ac_kernel<<<grid, block, smem, st>>>(L);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -481,7 +488,8 @@ cudaError_t prepare_exact_kernels(int max_smem) {
                          (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_FP64>,
                          (const void*)SP_KERNEL_NS::transient_fixed_kernel,
                          (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT, false>,
-                         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT, true>, (const void*)ac_kernel,
+                         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64_EXACT, true>, (const void*)ac_kernel, (const void*)ac_values_kernel,
+                         (const void*)ac_sparse_kernel,
                          (const void*)lu_batch_fp64_kernel, (const void*)lu_batch_cta_kernel<false>};
     for (const void* f : fns) {
         cudaError_t e = allow_dynamic_smem(f, max_smem);
