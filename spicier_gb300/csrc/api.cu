@@ -1288,6 +1288,7 @@ static int grid_locked(sp_ctx* ctx, const sp_grid_config* c, uint64_t seed, uint
     L.count = count;
     L.ws = (char*)ctx->scratch + extra;
     L.ws_stride = W.total;
+    L.max_smem = ctx->max_smem;
     L.x = d_x;
     L.newton = d_newton;
     L.krylov = d_krylov;

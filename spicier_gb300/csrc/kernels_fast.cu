@@ -12,6 +12,7 @@
 #include "ladder.cuh"
 #include "transient_fixed.cuh"
 #include "powergrid.cuh"
+#include "powergrid_mixed.cuh"
 #include <algorithm>
 
 namespace sp {
@@ -564,10 +565,14 @@ cudaError_t launch_yield(const double* v, uint64_t rows, uint32_t ld, const uint
 }
 
 cudaError_t launch_grid(const GridLaunch& L, int precision, cudaStream_t st) {
-    if (precision == SP_PREC_MIXED)
-        SP_KERNEL_NS::grid_kernel<SP_PREC_MIXED><<<(unsigned)L.count, kGridThreads, grid_smem_bytes(L.cfg, 4), st>>>(L);
-    else
-        SP_KERNEL_NS::grid_kernel<SP_PREC_FP64><<<(unsigned)L.count, kGridThreads, grid_smem_bytes(L.cfg, 8), st>>>(L);
+    if (precision == SP_PREC_MIXED) {
+        const int n = L.cfg.rows * L.cfg.cols + 1, nq = grid_mixed_rows(n);
+        auto kernel = nq == 2 ? SP_KERNEL_NS::grid_mixed_kernel<2>
+                              : (nq == 4 ? SP_KERNEL_NS::grid_mixed_kernel<4> : SP_KERNEL_NS::grid_mixed_kernel<8>);
+        kernel<<<(unsigned)L.count, kGridMixedThreads, grid_mixed_smem(n, L.cfg.restart, L.max_smem).total, st>>>(L);
+    } else {
+        SP_KERNEL_NS::grid_kernel<<<(unsigned)L.count, kGridThreads, grid_smem_bytes(L.cfg, 8), st>>>(L);
+    }
     return cudaGetLastError();
 }
 
@@ -579,7 +584,8 @@ cudaError_t launch_transient_fast(const TransientLaunch& L, int block, size_t sm
 
 cudaError_t prepare_fast_kernels(int max_smem) {
     const void* fns[] = {
-        (const void*)SP_KERNEL_NS::grid_kernel<SP_PREC_MIXED>, (const void*)SP_KERNEL_NS::grid_kernel<SP_PREC_FP64>,
+        (const void*)SP_KERNEL_NS::grid_kernel, (const void*)SP_KERNEL_NS::grid_mixed_kernel<2>,
+        (const void*)SP_KERNEL_NS::grid_mixed_kernel<4>, (const void*)SP_KERNEL_NS::grid_mixed_kernel<8>,
         (const void*)SP_KERNEL_NS::transient_fixed_kernel, (const void*)ac_mixed_kernel,
         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED, false>, (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED, true>,
         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64, false>, (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64, true>,

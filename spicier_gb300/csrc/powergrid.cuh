@@ -35,6 +35,7 @@ struct GridLaunch {
     uint64_t seed, first, count;
     void* ws;          // per instance: ws + i * ws_stride bytes
     size_t ws_stride;  // bytes
+    int max_smem;      // dynamic shared memory a block may have
     double* x;         // [count][n]
     int32_t* newton;
     int32_t* krylov;
@@ -78,7 +79,8 @@ __host__ __device__ inline size_t grid_smem_bytes(const sp_grid_config& c, int t
 #ifdef SP_KERNEL_NS
 namespace SP_KERNEL_NS {
 
-// Block maximum (order-free).
+// Maximum over the first T threads (order-free).
+template <int T = kGridThreads>
 __device__ inline double block_max(double v, double* red) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -86,7 +88,7 @@ __device__ inline double block_max(double v, double* red) {
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
     double m = 0.0;
-    for (int w = 0; w < kGridThreads / 32; ++w) m = fmax(m, red[w]);
+    for (int w = 0; w < T / 32; ++w) m = fmax(m, red[w]);
     __syncthreads();
     return m;
 }
@@ -135,9 +137,169 @@ __device__ inline T grid_apply_row(const sp_grid_config& c, const double* gh, co
     return v;
 }
 
-template <int PREC>
+// Rows (and sinks) of thread t start at t and are T apart; threads past the first T own none.
+template <int T>
+__device__ inline int grid_first(int none) {
+    return threadIdx.x < T ? (int)threadIdx.x : none;
+}
+
+// Pointers into one instance's workspace.
+struct GridPtrs {
+    double *gh, *gv, *diag, *b, *r, *vgs, *sids, *sgds;
+    int* sink;
+    unsigned char* V;
+};
+
+__device__ inline GridPtrs grid_ptrs(const GridLaunch& L, const GridWs& W, uint32_t i) {
+    unsigned char* base = (unsigned char*)L.ws + (size_t)i * L.ws_stride;
+    GridPtrs g;
+    g.gh = (double*)(base + W.gh);
+    g.gv = (double*)(base + W.gv);
+    g.diag = (double*)(base + W.diag);
+    g.b = (double*)(base + W.b);
+    g.r = (double*)(base + W.r);
+    g.sink = (int*)(base + W.sink);
+    g.vgs = (double*)(base + W.vgs);
+    g.sids = (double*)(base + W.sids);
+    g.sgds = (double*)(base + W.sgds);
+    g.V = base + W.V;
+    return g;
+}
+
+// The instance's draws, in the oracle's order (edges horizontal, vertical;
+// sinks node, VGS), and x = 0.  Ends with a barrier.
+template <int T>
+__device__ inline void grid_draws(const GridLaunch& L, const GridPtrs& g, uint32_t inst, double* x) {
+    const sp_grid_config& c = L.cfg;
+    const int nn = c.rows * c.cols;
+    const uint32_t layout = inst / 4, corner = inst % 4;
+    const double scale = (corner & 1) ? c.r_scale_hi : c.r_scale_lo;
+    unsigned hard = 0;
+    const double lr = cr_log(c.r_hi / c.r_lo, &hard);
+    const int nh = c.rows * (c.cols - 1), nv = (c.rows - 1) * c.cols;
+    for (int e = grid_first<T>(nh + nv); e < nh + nv; e += T) {
+        const double u = rng_uniform(L.seed, layout, (uint32_t)e);
+        const double cond = 1.0 / (c.r_lo * cr_exp(u * lr, &hard) * scale);
+        if (e < nh) g.gh[e] = cond;
+        else g.gv[e - nh] = cond;
+    }
+    for (int s = grid_first<T>(c.num_sinks); s < c.num_sinks; s += T) {
+        const uint32_t idx = (uint32_t)(nh + nv + 2 * s);
+        g.sink[s] = (int)floor((double)nn * rng_uniform(L.seed, layout, idx));
+        g.vgs[s] = c.vgs_lo + rng_uniform(L.seed, layout, idx + 1) * (c.vgs_hi - c.vgs_lo);
+    }
+    for (int p = grid_first<T>(nn + 1); p <= nn; p += T) x[p] = 0.0;
+    __syncthreads();
+}
+
+__device__ inline double grid_vto(const sp_grid_config& c, uint32_t inst) {
+    return (inst % 4 & 2) ? c.vto + c.vto_shift : c.vto - c.vto_shift;
+}
+
+// Diagonal and right-hand side of the system linearised at x.  Each node's
+// sinks are added in sink order by the node's owner, which walks the whole
+// list (one walker took 512 dependent round trips to memory per iteration).
+// Ends without a barrier: rows of diag and b belong to their thread.
+template <int T>
+__device__ inline void grid_linearise(const sp_grid_config& c, const GridPtrs& g, double vto, double beta,
+                                      const double* x) {
+    const int nn = c.rows * c.cols, n = nn + 1, tid = threadIdx.x;
+    for (int s = grid_first<T>(c.num_sinks); s < c.num_sinks; s += T) {
+        const double vds = x[g.sink[s]], vg = g.vgs[s], vth = fabs(vto);
+        double ids, gds;
+        if (vg < vth) {
+            ids = 0.0;
+            gds = 1e-12;
+        } else if (vds < vg - vth) {
+            const double vov = vg - vth;
+            ids = beta * (vov * vds - 0.5 * vds * vds) * (1.0 + c.lambda * vds);
+            gds = fmax(beta * (vov - vds) * (1.0 + c.lambda * vds) + beta * (vov * vds - 0.5 * vds * vds) * c.lambda,
+                       1e-12);
+        } else {
+            const double vov = vg - vth;
+            ids = 0.5 * beta * vov * vov * (1.0 + c.lambda * vds);
+            gds = fmax(0.5 * beta * vov * vov * c.lambda, 1e-12);
+        }
+        g.sids[s] = ids - gds * vds;
+        g.sgds[s] = gds;
+    }
+    for (int p = grid_first<T>(n); p < n; p += T) {
+        double d = 0.0;
+        if (p < nn) {
+            const int rr = p / c.cols, j = p - rr * c.cols;
+            if (j > 0) d += g.gh[rr * (c.cols - 1) + j - 1];
+            if (j < c.cols - 1) d += g.gh[rr * (c.cols - 1) + j];
+            if (rr > 0) d += g.gv[(rr - 1) * c.cols + j];
+            if (rr < c.rows - 1) d += g.gv[rr * c.cols + j];
+            if (p == 0) d += 3.0 * c.strap_g;
+            else if (p == c.cols - 1 || p == (c.rows - 1) * c.cols || p == nn - 1) d += c.strap_g;
+        }
+        g.diag[p] = d;
+        g.b[p] = p < nn ? 0.0 : c.vdd;
+    }
+    __syncthreads();
+    if (tid < T) {
+#pragma unroll 4
+        for (int s = 0; s < c.num_sinks; ++s) {
+            const int p = g.sink[s];
+            if ((p & (T - 1)) == tid) {
+                g.diag[p] += g.sgds[s];
+                g.b[p] -= g.sids[s];
+            }
+        }
+    }
+}
+
+// KCL residual at the final iterate (FP64): the largest |A(x) x - b(x)| of the node rows.
+template <int T>
+__device__ inline double grid_residual(const sp_grid_config& c, const GridPtrs& g, double vto, double beta,
+                                       const double* x, double* redd) {
+    const int nn = c.rows * c.cols, tid = threadIdx.x;
+    for (int s = grid_first<T>(c.num_sinks); s < c.num_sinks; s += T) {
+        const double vds = x[g.sink[s]], vg = g.vgs[s], vth = fabs(vto);
+        double ids;
+        if (vg < vth) ids = 0.0;
+        else if (vds < vg - vth) {
+            const double vov = vg - vth;
+            ids = beta * (vov * vds - 0.5 * vds * vds) * (1.0 + c.lambda * vds);
+        } else {
+            const double vov = vg - vth;
+            ids = 0.5 * beta * vov * vov * (1.0 + c.lambda * vds);
+        }
+        g.sids[s] = ids;
+    }
+    for (int p = grid_first<T>(nn); p < nn; p += T) {
+        const int rr = p / c.cols, j = p - rr * c.cols;
+        double v = 0.0;  // currents leaving node p through the grid and straps
+        if (j > 0) v += g.gh[rr * (c.cols - 1) + j - 1] * (x[p] - x[p - 1]);
+        if (j < c.cols - 1) v += g.gh[rr * (c.cols - 1) + j] * (x[p] - x[p + 1]);
+        if (rr > 0) v += g.gv[(rr - 1) * c.cols + j] * (x[p] - x[p - c.cols]);
+        if (rr < c.rows - 1) v += g.gv[rr * c.cols + j] * (x[p] - x[p + c.cols]);
+        if (p == 0) {
+            v += c.strap_g * (x[0] - x[c.cols - 1]);
+            v += c.strap_g * (x[0] - x[(c.rows - 1) * c.cols]);
+            v += c.strap_g * (x[0] - x[nn - 1]);
+            v += x[nn];
+        } else if (p == c.cols - 1 || p == (c.rows - 1) * c.cols || p == nn - 1) {
+            v += c.strap_g * (x[p] - x[0]);
+        }
+        g.r[p] = v;
+    }
+    __syncthreads();
+    if (tid < T) {
+#pragma unroll 4
+        for (int s = 0; s < c.num_sinks; ++s) {
+            const int p = g.sink[s];
+            if ((p & (T - 1)) == tid) g.r[p] += g.sids[s];
+        }
+    }
+    double mx = 0.0;
+    for (int p = grid_first<T>(nn); p < nn; p += T) mx = fmax(mx, fabs(g.r[p]));
+    return block_max<T>(mx, redd);
+}
+
 __global__ void __launch_bounds__(kGridThreads, 1) grid_kernel(GridLaunch L) {
-    using T = typename std::conditional<PREC == SP_PREC_MIXED, float, double>::type;
+    using T = double;
     extern __shared__ __align__(16) unsigned char gsm[];
     const sp_grid_config& c = L.cfg;
     const int n = c.rows * c.cols + 1, nn = n - 1, m = c.restart;
@@ -145,17 +307,9 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_kernel(GridLaunch L) {
     const uint32_t i = blockIdx.x;
     const uint32_t inst = (uint32_t)(L.first + i);
     const GridWs W = grid_ws(c, (int)sizeof(T));
-    unsigned char* base = (unsigned char*)L.ws + (size_t)i * L.ws_stride;
-    double* gh = (double*)(base + W.gh);
-    double* gv = (double*)(base + W.gv);
-    double* diag = (double*)(base + W.diag);
-    double* b = (double*)(base + W.b);
-    double* r = (double*)(base + W.r);
-    int* sink = (int*)(base + W.sink);
-    double* vgs = (double*)(base + W.vgs);
-    double* sids = (double*)(base + W.sids);
-    double* sgds = (double*)(base + W.sgds);
-    T* V = (T*)(base + W.V);
+    const GridPtrs g = grid_ptrs(L, W, i);
+    double *gh = g.gh, *gv = g.gv, *diag = g.diag, *b = g.b, *r = g.r;
+    T* V = (T*)g.V;
     // shared: z (the vector multiplied, T), Jacobi inverse in T, small dense parts
     T* zs = reinterpret_cast<T*>(gsm);
     T* inv = zs + n;
@@ -171,127 +325,33 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_kernel(GridLaunch L) {
     T* hcol = proj + (kGridThreads / 32) * (kGridMaxRestart + 1);
     double* x = L.x + (size_t)i * n;
 
-    // --- draws (the oracle's order: edges horizontal, vertical; sinks node, VGS)
-    const uint32_t layout = inst / 4, corner = inst % 4;
-    const double scale = (corner & 1) ? c.r_scale_hi : c.r_scale_lo;
-    const double vto = (corner & 2) ? c.vto + c.vto_shift : c.vto - c.vto_shift;
-    unsigned hard = 0;
-    const double lr = cr_log(c.r_hi / c.r_lo, &hard);
-    const int nh = c.rows * (c.cols - 1), nv = (c.rows - 1) * c.cols;
-    for (int e = tid; e < nh + nv; e += kGridThreads) {
-        const double u = rng_uniform(L.seed, layout, (uint32_t)e);
-        const double g = 1.0 / (c.r_lo * cr_exp(u * lr, &hard) * scale);
-        if (e < nh) gh[e] = g;
-        else gv[e - nh] = g;
-    }
-    for (int s = tid; s < c.num_sinks; s += kGridThreads) {
-        const uint32_t idx = (uint32_t)(nh + nv + 2 * s);
-        sink[s] = (int)floor((double)nn * rng_uniform(L.seed, layout, idx));
-        vgs[s] = c.vgs_lo + rng_uniform(L.seed, layout, idx + 1) * (c.vgs_hi - c.vgs_lo);
-    }
-    for (int p = tid; p < n; p += kGridThreads) x[p] = 0.0;
-    __syncthreads();
+    grid_draws<kGridThreads>(L, g, inst, x);
+    const double vto = grid_vto(c, inst);
 
     int newton_it = 0, krylov_total = 0;
     uint8_t status = SP_ST_FAILED;
     double resid = 0.0;
     const double beta = c.kp * 1.0 * c.w / c.l;  // level1.rs:68-70 (NF = 1)
     for (int it = 1; it <= c.max_newton; ++it) {
-        // --- linearise at x: sinks in parallel, accumulated in sink order by thread 0
-        for (int s = tid; s < c.num_sinks; s += kGridThreads) {
-            const double vds = x[sink[s]], vg = vgs[s], vth = fabs(vto);
-            double ids, gds;
-            if (vg < vth) {
-                ids = 0.0;
-                gds = 1e-12;
-            } else if (vds < vg - vth) {
-                const double vov = vg - vth;
-                ids = beta * (vov * vds - 0.5 * vds * vds) * (1.0 + c.lambda * vds);
-                gds = fmax(beta * (vov - vds) * (1.0 + c.lambda * vds) + beta * (vov * vds - 0.5 * vds * vds) * c.lambda,
-                           1e-12);
-            } else {
-                const double vov = vg - vth;
-                ids = 0.5 * beta * vov * vov * (1.0 + c.lambda * vds);
-                gds = fmax(0.5 * beta * vov * vov * c.lambda, 1e-12);
-            }
-            sids[s] = ids - gds * vds;
-            sgds[s] = gds;
-        }
-        for (int p = tid; p < n; p += kGridThreads) {
-            double d = 0.0;
-            if (p < nn) {
-                const int rr = p / c.cols, j = p - rr * c.cols;
-                if (j > 0) d += gh[rr * (c.cols - 1) + j - 1];
-                if (j < c.cols - 1) d += gh[rr * (c.cols - 1) + j];
-                if (rr > 0) d += gv[(rr - 1) * c.cols + j];
-                if (rr < c.rows - 1) d += gv[rr * c.cols + j];
-                if (p == 0) d += 3.0 * c.strap_g;
-                else if (p == c.cols - 1 || p == (c.rows - 1) * c.cols || p == nn - 1) d += c.strap_g;
-            }
-            diag[p] = d;
-            b[p] = p < nn ? 0.0 : c.vdd;
-        }
-        __syncthreads();
-        if (tid == 0)
-            for (int s = 0; s < c.num_sinks; ++s) {
-                diag[sink[s]] += sgds[s];
-                b[sink[s]] -= sids[s];
-            }
-        __syncthreads();
+        grid_linearise<kGridThreads>(c, g, vto, beta, x);
         for (int p = tid; p < n; p += kGridThreads) {
             inv[p] = (T)(fabs(diag[p]) < 1e-30 ? 1.0 : 1.0 / diag[p]);
             dT[p] = (T)diag[p];
         }
-        // --- right-hand side of the Krylov solve: b (FP64 mode) or b - A x (mixed)
-        if (PREC == SP_PREC_MIXED) {
-            for (int p = tid; p < n; p += kGridThreads) zs[p] = (T)0;
-            __syncthreads();
-            // residual in FP64 from x in global memory
-            for (int p = tid; p < n; p += kGridThreads) {
-                double v;
-                if (p == nn) {
-                    v = x[0];
-                } else {
-                    const int rr = p / c.cols, j = p - rr * c.cols;
-                    v = diag[p] * x[p];
-                    if (j > 0) v -= gh[rr * (c.cols - 1) + j - 1] * x[p - 1];
-                    if (j < c.cols - 1) v -= gh[rr * (c.cols - 1) + j] * x[p + 1];
-                    if (rr > 0) v -= gv[(rr - 1) * c.cols + j] * x[p - c.cols];
-                    if (rr < c.rows - 1) v -= gv[rr * c.cols + j] * x[p + c.cols];
-                    if (p == 0) {
-                        v -= c.strap_g * x[c.cols - 1];
-                        v -= c.strap_g * x[(c.rows - 1) * c.cols];
-                        v -= c.strap_g * x[nn - 1];
-                        v += x[nn];
-                    } else if (p == c.cols - 1 || p == (c.rows - 1) * c.cols || p == nn - 1) {
-                        v -= c.strap_g * x[0];
-                    }
-                }
-                r[p] = b[p] - v;
-            }
-        } else {
-            for (int p = tid; p < n; p += kGridThreads) r[p] = b[p];
-        }
+        for (int p = tid; p < n; p += kGridThreads) r[p] = b[p];
         __syncthreads();
-        // the KCL residual of the mixed path's current iterate decides convergence too
-        double rmax = 0.0;
-        if (PREC == SP_PREC_MIXED)
-            for (int p = tid; p < nn; p += kGridThreads) rmax = fmax(rmax, fabs(r[p]));
-        // --- GMRES on A d = r (d accumulated into r's solution vector sol)
+        // --- GMRES on A x_new = b
         // sol lives in b's storage after this point (b is no longer needed)
         double* sol = b;
         for (int p = tid; p < n; p += kGridThreads) sol[p] = 0.0;
         T rnorm2_local = 0;
         for (int p = tid; p < n; p += kGridThreads) rnorm2_local += (T)r[p] * (T)r[p];
         const double b_norm = sqrt((double)block_sum<T>(rnorm2_local, red));
-        // FP32 Krylov: each solve only has to gain three digits; the FP64
-        // residual of the next Newton iteration refines the rest
-        const double tol = PREC == SP_PREC_MIXED ? fmax(c.krylov_tol, 1e-3) : c.krylov_tol;
+        const double tol = c.krylov_tol;
         int total = 0;
         bool solved = b_norm < 1e-30;
         for (int cycle = 0; !solved && cycle < c.max_krylov; ++cycle) {
-            // residual of the current solution, r - A sol, in FP64 (an FP32
-            // difference of two nearly equal vectors would stall the restarts)
+            // residual of the current solution, r - A sol
             __syncthreads();
             T loc = 0;
             for (int p = tid; p < n; p += kGridThreads) {
@@ -441,7 +501,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_kernel(GridLaunch L) {
         bool ok = true, fin = true;
         for (int p = tid; p < n; p += kGridThreads) {
             const double old = x[p];
-            const double nw = PREC == SP_PREC_MIXED ? old + sol[p] : sol[p];
+            const double nw = sol[p];
             const double tl = c.v_reltol * fmax(fabs(nw), fabs(old)) + (p < nn ? c.v_abstol : c.i_abstol);
             ok = ok && fabs(nw - old) <= tl;
             fin = fin && isfinite(nw);
@@ -450,11 +510,6 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_kernel(GridLaunch L) {
         ok = __syncthreads_and(ok);
         fin = __syncthreads_and(fin);
         newton_it = it;
-        if (PREC == SP_PREC_MIXED) {
-            // rmax is the KCL residual before this update: converged when the
-            // step test passes and that residual already met the target
-            ok = ok && block_max(rmax, redd) <= c.resid_target;
-        }
         if (!fin) {
             status = SP_ST_NONFINITE;
             break;
@@ -464,44 +519,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) grid_kernel(GridLaunch L) {
             break;
         }
     }
-    // --- KCL residual at the final iterate (FP64): A(x) x - b(x), node rows
-    for (int s = tid; s < c.num_sinks; s += kGridThreads) {
-        const double vds = x[sink[s]], vg = vgs[s], vth = fabs(vto);
-        double ids;
-        if (vg < vth) ids = 0.0;
-        else if (vds < vg - vth) {
-            const double vov = vg - vth;
-            ids = beta * (vov * vds - 0.5 * vds * vds) * (1.0 + c.lambda * vds);
-        } else {
-            const double vov = vg - vth;
-            ids = 0.5 * beta * vov * vov * (1.0 + c.lambda * vds);
-        }
-        sids[s] = ids;
-    }
-    for (int p = tid; p < nn; p += kGridThreads) {
-        const int rr = p / c.cols, j = p - rr * c.cols;
-        double v = 0.0;  // currents leaving node p through the grid and straps
-        if (j > 0) v += gh[rr * (c.cols - 1) + j - 1] * (x[p] - x[p - 1]);
-        if (j < c.cols - 1) v += gh[rr * (c.cols - 1) + j] * (x[p] - x[p + 1]);
-        if (rr > 0) v += gv[(rr - 1) * c.cols + j] * (x[p] - x[p - c.cols]);
-        if (rr < c.rows - 1) v += gv[rr * c.cols + j] * (x[p] - x[p + c.cols]);
-        if (p == 0) {
-            v += c.strap_g * (x[0] - x[c.cols - 1]);
-            v += c.strap_g * (x[0] - x[(c.rows - 1) * c.cols]);
-            v += c.strap_g * (x[0] - x[nn - 1]);
-            v += x[nn];
-        } else if (p == c.cols - 1 || p == (c.rows - 1) * c.cols || p == nn - 1) {
-            v += c.strap_g * (x[p] - x[0]);
-        }
-        r[p] = v;
-    }
-    __syncthreads();
-    if (tid == 0)
-        for (int s = 0; s < c.num_sinks; ++s) r[sink[s]] += sids[s];
-    __syncthreads();
-    double mx = 0.0;
-    for (int p = tid; p < nn; p += kGridThreads) mx = fmax(mx, fabs(r[p]));
-    resid = block_max(mx, redd);
+    resid = grid_residual<kGridThreads>(c, g, vto, beta, x, redd);
     if (tid == 0) {
         L.newton[i] = newton_it;
         L.krylov[i] = krylov_total;
