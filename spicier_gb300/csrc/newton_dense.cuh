@@ -729,7 +729,9 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
     const bool warm = L.x0 != nullptr || L.lin != nullptr;  // listed samples started warm
     const unsigned int misses = *L.fail_count;
     const SoACg dv{L.dv.p, L.dv.stride};
-    for (unsigned int j = blockIdx.x * blockDim.x + threadIdx.x; j < misses; j += gridDim.x * blockDim.x) {
+    // neighbours in the list go to different blocks: chains differ in length at
+    // every level, and lanes of one warp wait for each other there
+    for (unsigned int j = threadIdx.x * gridDim.x + blockIdx.x; j < misses; j += gridDim.x * blockDim.x) {
         const size_t s = L.fail_list[j];
         if (L.redraw.derived) redraw_sample(L.c, L.redraw, L.dv.stride, s);
         int total = L.iters ? L.iters[s] : 0;
