@@ -112,9 +112,18 @@ __host__ __device__ inline void mos_eval(bool pmos, double vth, double beta, dou
         gm = 0.0;
     } else if (below(vds, vgs - vth)) {
         double vov = vgs - vth;
+#if defined(__CUDA_ARCH__) && !defined(SP_EXACT_UNIT)
+        // fused as the compiler did in most kernels: left to it, the choice differs
+        // from one kernel to the next, and with it the bits of a sample that one
+        // kernel takes over from another
+        double half = fma(vov, vds, -(0.5 * vds * vds)), q = fma(lambda, vds, 1.0);
+        double i = beta * half * q;
+        double g = fma(beta * half, lambda, beta * (vov - vds) * q);
+#else
         double i = beta * (vov * vds - 0.5 * vds * vds) * (1.0 + lambda * vds);
         double g = beta * (vov - vds) * (1.0 + lambda * vds) +
                    beta * (vov * vds - 0.5 * vds * vds) * lambda;
+#endif
         double m = beta * vds * (1.0 + lambda * vds);
         ids = pmos ? -i : i;
         gds = fmax(g, 1e-12);
