@@ -430,7 +430,10 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     size_t be = align256(sizeof(sp_element) * c->num_elements);
     size_t bp = align256(sizeof(sp_param) * c->num_params);
     size_t bu = align256(sizeof(sp_pulse) * c->num_pulses);
-    size_t bo = align256(sizeof(int) * c->num_elements);
+    std::vector<int> b3;  // BSIM3 devices, kept behind the offsets
+    for (int e = 0; e < c->num_elements; ++e)
+        if (c->elements[e].kind == SP_EL_BSIM3N || c->elements[e].kind == SP_EL_BSIM3P) b3.push_back(e);
+    size_t bo = align256(sizeof(int) * (c->num_elements + b3.size()));
     size_t bn = align256(sizeof(double) * t->n);
     std::vector<int> drawn;
     for (int k = 0; k < c->num_params; ++k)
@@ -525,6 +528,8 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
         e = cudaMemcpy(dpul, c->pulses, sizeof(sp_pulse) * c->num_pulses, cudaMemcpyHostToDevice);
     if (e == cudaSuccess && c->num_elements)
         e = cudaMemcpy(ddoff, doff.data(), sizeof(int) * c->num_elements, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !b3.empty())
+        e = cudaMemcpy(ddoff + c->num_elements, b3.data(), sizeof(int) * b3.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && c->nodeset) e = cudaMemcpy(dns, c->nodeset, sizeof(double) * t->n, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(t->dev);
@@ -532,7 +537,7 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
         return cuda_fail(ctx, e, "topology upload");
     }
     t->dc = DevCircuit{c->num_nodes, c->num_branches, t->n, c->num_elements, c->num_params, nd,
-                       del, dpar, dpul, ddoff, c->nodeset ? dns : nullptr};
+                       del, dpar, dpul, ddoff, c->nodeset ? dns : nullptr, ddoff + c->num_elements, (int)b3.size()};
     t->d_tran = dtran;
     t->d_gauss32 = dgauss;
     t->d_ac = dac;
@@ -762,7 +767,20 @@ static int newton_dc_locked(sp_ctx* ctx, const sp_topology* t, const sp_newton_c
     const int kprec = prec == SP_PREC_MIXED ? SP_PREC_MIXED : SP_PREC_FP64;
     size_t per = kprec == SP_PREC_MIXED ? work_bytes_per_thread<SP_PREC_MIXED>(t->n)
                                         : work_bytes_per_thread<SP_PREC_FP64>(t->n);
-    int block = pick_block(per, ctx->max_smem, count, ctx->num_sms);
+    // The BSIM3 devices of a sample go to the lanes of a team: an evaluation is
+    // about 350 FP64 instructions of 64 cycles each, however few lanes take part.
+    // In the primary kernel that pays while single lanes would leave quarters of
+    // SMs without a warp (three devices: 2,000 samples 5.7 -> 4.6 ms, 8,192
+    // 6.6 -> 6.1, but 12,000 6.4 -> 7.8, a call with its fallback); the fallback
+    // decides by the length of its list (8,192 samples, 169 of them listed: 6.7
+    // -> 3.4 ms).
+    int team = 1;
+    while (team < 8 && team < t->dc.num_b3) team *= 2;
+    if (prec == SP_PREC_FP64_EXACT) team = 1;  // (no instances of those kernels)
+    L.fallback_team = team;
+    if (!use_spec && count * team <= (uint64_t)ctx->num_sms * 32 * 7) L.team = team;
+    const uint64_t lanes = count * L.team;
+    int block = pick_block(per, ctx->max_smem, lanes, ctx->num_sms);
     if (!block) return fail(ctx, SP_ERR_INVALID_DIMENSION, "MNA size %d does not fit shared memory", t->n);
     {
         // tuned threads per block (setting "newton.block.<precision>"), within what shared memory allows
@@ -771,7 +789,7 @@ static int newton_dc_locked(sp_ctx* ctx, const sp_topology* t, const sp_newton_c
         if (tb >= 32 && tb % 32 == 0 && tb <= 1024 && per * tb <= (size_t)ctx->max_smem) block = tb;
     }
     size_t smem = per * block;
-    int grid = (int)((count + block - 1) / block);
+    int grid = (int)((lanes + block - 1) / block);
     // Placed while the draw kernel drains, blocks crowd onto the SMs that finish
     // first.  A grid of a few blocks per SM asks for so much shared memory that
     // no SM can take more than its share (and the fallback's blocks still fit):

@@ -59,6 +59,8 @@ struct DevCircuit {
     const sp_pulse* pulses;  // [num_pulses]
     const int* doff;         // [num_elements] offset of each element's derived block
     const double* nodeset;   // [n] or nullptr
+    const int* b3 = nullptr;  // [num_b3] elements that are BSIM3 devices, in order
+    int num_b3 = 0;
 };
 
 // Thermal voltage at 300.15 K, k*T/q with CODATA constants (diode.rs:41-45).
@@ -460,6 +462,43 @@ struct sink_int_tests<S, typename std::enable_if<S::kIntTests>::type> {
     static constexpr bool value = true;
 };
 
+// Sinks that declare kTeam have `team` lanes (a power of two) that stamp the
+// same sample together, each evaluating its share of the BSIM3 devices.
+template <class S, class = void>
+struct sink_team {
+    static constexpr bool value = false;
+};
+template <class S>
+struct sink_team<S, typename std::enable_if<S::kTeam>::type> {
+    static constexpr bool value = true;
+};
+
+#if defined(__CUDACC__)
+// bsim3_eval of device `nth` (element e) at its terminal voltages, by the lane
+// of the team whose turn it is; `mine` holds this lane's result of the latest
+// `team` devices.
+template <class DV, class Sink>
+__device__ inline Bsim3Out bsim3_eval_team(const DevCircuit& c, const DV& dv, size_t s, const Sink& k, int nth,
+                                           Bsim3Out& mine) {
+    const int team = k.team, turn = nth & (team - 1);
+    if (turn == 0) {
+        const int at = nth + (int)(threadIdx.x & (team - 1)), e = c.b3[at < c.num_b3 ? at : c.num_b3 - 1];
+        const sp_element el = c.el[e];
+        const int off = c.doff[e];
+        const double vg = el.node[1] >= 0 ? k.x(el.node[1]) : 0.0, vd = el.node[0] >= 0 ? k.x(el.node[0]) : 0.0;
+        const double vs = el.node[2] >= 0 ? k.x(el.node[2]) : 0.0, vb = el.node[3] >= 0 ? k.x(el.node[3]) : 0.0;
+        mine = bsim3_eval(el.kind == SP_EL_BSIM3P, [&](int i) { return dv(off + i, s); }, vg - vs, vd - vs, vb - vs);
+    }
+    const unsigned lanes = (team == 32 ? 0xffffffffu : (1u << team) - 1u) << (threadIdx.x & 31 & -team);
+    Bsim3Out r;
+    r.ids = __shfl_sync(lanes, mine.ids, turn, team);
+    r.gds = __shfl_sync(lanes, mine.gds, turn, team);
+    r.gm = __shfl_sync(lanes, mine.gm, turn, team);
+    r.gmbs = __shfl_sync(lanes, mine.gmbs, turn, team);
+    return r;
+}
+#endif
+
 // Stamps of a Level-1 MOSFET, in the reference's order; a sink may bring its own.
 template <class Sink>
 __host__ __device__ inline void stamp_mos(Sink& k, int d, int g, int so, double gds, double gm, double ieq) {
@@ -488,6 +527,8 @@ template <class DV, class Sink>
 __host__ __device__ inline void stamp_all(const DevCircuit& c, const DV& dv, size_t s, Sink& k, int mode,
                                  double aux) {
     const bool scaled = (mode == STAMP_SCALED);
+    [[maybe_unused]] int b3 = 0;  // BSIM3 devices so far (teams)
+    [[maybe_unused]] Bsim3Out b3_mine;
     for (int e = 0; e < c.num_elements; ++e) {
         const sp_element el = c.el[e];
         const int off = c.doff[e];
@@ -644,8 +685,11 @@ __host__ __device__ inline void stamp_all(const DevCircuit& c, const DV& dv, siz
                 const double vs = so >= 0 ? k.x(so) : 0.0;
                 const double vb = b >= 0 ? k.x(b) : 0.0;
                 const double vgs = vg - vs, vds = vd - vs, vbs = vb - vs;
-                const Bsim3Out r = bsim3_eval(el.kind == SP_EL_BSIM3P, [&](int i) { return dv(off + i, s); },
-                                              vgs, vds, vbs);
+                Bsim3Out r;
+                if constexpr (sink_team<Sink>::value)
+                    r = bsim3_eval_team(c, dv, s, k, b3++, b3_mine);
+                else
+                    r = bsim3_eval(el.kind == SP_EL_BSIM3P, [&](int i) { return dv(off + i, s); }, vgs, vds, vbs);
                 if (d >= 0) k.add(d, d, r.gds);
                 if (so >= 0) k.add(so, so, r.gds);
                 if (d >= 0 && so >= 0) {

@@ -21,11 +21,14 @@ cudaError_t launch_newton_fast(int prec, const NewtonLaunch& L, bool fallback, i
                                size_t smem, cudaStream_t st) {
     using namespace SP_KERNEL_NS;
     const dim3 g(grid), b(block);
-    if (prec == SP_PREC_MIXED)
-        return fallback ? launch_chained(newton_fallback_kernel<SP_PREC_MIXED>, g, b, smem, st, L)
-                        : launch_chained(newton_primary_kernel<SP_PREC_MIXED>, g, b, smem, st, L);
-    return fallback ? launch_chained(newton_fallback_kernel<SP_PREC_FP64>, g, b, smem, st, L)
-                    : launch_chained(newton_primary_kernel<SP_PREC_FP64>, g, b, smem, st, L);
+    static void (*const kernels[2][2][2])(NewtonLaunch) = {  // [mixed][fallback][team]
+        {{newton_primary_kernel<SP_PREC_FP64>, newton_primary_kernel<SP_PREC_FP64, true>},
+         {newton_fallback_kernel<SP_PREC_FP64>, newton_fallback_kernel<SP_PREC_FP64, true>}},
+        {{newton_primary_kernel<SP_PREC_MIXED>, newton_primary_kernel<SP_PREC_MIXED, true>},
+         {newton_fallback_kernel<SP_PREC_MIXED>, newton_fallback_kernel<SP_PREC_MIXED, true>}}};
+    const bool team = (fallback ? L.fallback_team : L.team) > 1;
+    auto kernel = kernels[prec == SP_PREC_MIXED][fallback][team];
+    return launch_chained(kernel, g, b, smem, st, L);
 }
 
 // Mixed-precision BatchedLuSolver::solve_batch: FP32 partial-pivot LU in
@@ -589,6 +592,8 @@ cudaError_t prepare_fast_kernels(int max_smem) {
         (const void*)SP_KERNEL_NS::transient_fixed_kernel, (const void*)ac_mixed_kernel,
         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED, false>, (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_MIXED, true>,
         (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64, false>, (const void*)SP_KERNEL_NS::ladder_kernel<SP_PREC_FP64, true>,
+        (const void*)SP_KERNEL_NS::newton_primary_kernel<SP_PREC_MIXED, true>, (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_MIXED, true>,
+        (const void*)SP_KERNEL_NS::newton_primary_kernel<SP_PREC_FP64, true>, (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_FP64, true>,
         (const void*)SP_KERNEL_NS::newton_primary_kernel<SP_PREC_MIXED>, (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_MIXED>,
         (const void*)SP_KERNEL_NS::newton_primary_kernel<SP_PREC_FP64>, (const void*)SP_KERNEL_NS::newton_fallback_kernel<SP_PREC_FP64>,
         (const void*)lu_batch_mixed_kernel, (const void*)lu_batch_escalate_kernel};

@@ -48,6 +48,7 @@ struct Il {  // interleaved per-thread array view
 };
 
 struct PlainSink {
+    static constexpr bool kTeam = false;
     Il<double> A, b, xs;
     int n;
     __device__ double x(int i) const { return xs[i]; }
@@ -59,6 +60,7 @@ struct PlainSink {
 // Jacobian in FP32, residual F = A x - b in FP64 (only one element writes a
 // branch row's RHS, so rhs_set is a subtraction from zero).
 struct MixedSink {
+    static constexpr bool kTeam = false;
     Il<float> J;
     Il<double> F, xs;
     int n;
@@ -72,6 +74,7 @@ struct MixedSink {
 };
 
 struct ResidSink {
+    static constexpr bool kTeam = false;
     Il<double> F, xs;
     __device__ double x(int i) const { return xs[i]; }
     __device__ void add(int r, int c, double v) { F[r] += v * xs[c]; }
@@ -105,6 +108,20 @@ struct MixedSinkRec : MixedSink {
         if (c == lane) rows |= 1u << r;
     }
 };
+
+// A sink, or (TEAM) the same for a sample that `team` lanes hold.
+template <class S>
+struct TeamSink : S {
+    static constexpr bool kTeam = true;
+    int team;
+    template <class... A>
+    __device__ TeamSink(int t, A... a) : S{a...}, team(t) {}
+};
+template <bool TEAM, class S, class... A>
+__device__ inline auto make_sink(int team, A... a) {
+    if constexpr (TEAM) return TeamSink<S>(team, a...);
+    else return S{a...};
+}
 
 // MOSFET stamps with their eight loads in flight together (one after the
 // other, each waits for the store before it) where no two entries coincide;
@@ -368,6 +385,7 @@ struct Work {
     Il<double> A;   // FP64 matrix [n*n]               (PREC FP64)
     Il<float> J;    // FP32 Jacobian [n*n]             (PREC MIXED)
     Il<float> d;    // FP32 RHS / step [n]             (PREC MIXED)
+    int team = 1;   // lanes that hold this sample, each in its own work area
 };
 
 template <int PREC>
@@ -406,7 +424,7 @@ __device__ inline bool step_ok(double old, double nw, double reltol, double abst
 }
 
 // One solve_newton_raphson from w.x; w.x holds the last iterate on return.
-template <int PREC, class DV>
+template <int PREC, bool TEAM = false, class DV>
 __device__ inline int newton_run(const DevCircuit& c, const DV& dv, size_t s,
                                  const sp_newton_config& cfg, int mode, double aux, Work& w,
                                  int& iters) {
@@ -416,7 +434,7 @@ __device__ inline int newton_run(const DevCircuit& c, const DV& dv, size_t s,
         if (PREC == SP_PREC_FP64) {
             for (int i = 0; i < n * n; ++i) w.A[i] = 0.0;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            PlainSink k{w.A, w.v, w.x, n};
+            auto k = make_sink<TEAM, PlainSink>(w.team, w.A, w.v, w.x, n);
             stamp_all(c, dv, s, k, mode, aux);
             if (!lu_solve_fp64(n, w.A, w.v)) {
                 iters = it + 1;
@@ -435,7 +453,7 @@ __device__ inline int newton_run(const DevCircuit& c, const DV& dv, size_t s,
         } else {
             for (int i = 0; i < n * n; ++i) w.J[i] = 0.0f;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            MixedSink k{w.J, w.v, w.x, n};
+            auto k = make_sink<TEAM, MixedSink>(w.team, w.J, w.v, w.x, n);
             stamp_all(c, dv, s, k, mode, aux);
             for (int i = 0; i < n; ++i) w.d[i] = (float)(-w.v[i]);
             if (!lu_solve_fp32(n, w.J, w.d)) {
@@ -470,7 +488,7 @@ __device__ inline bool step_ok_int(double old, double nw, double reltol, double 
 // the last one is done (active false: a lane without a sample, which follows
 // along on another's data).  *plain as in lu_solve_warp, cleared too where a
 // start point is not finite; the caller then repeats the lane with newton_run.
-template <int PREC>
+template <int PREC, bool TEAM>
 __device__ inline int newton_run_warp(const DevCircuit& c, const SoA& dv, size_t s, const sp_newton_config& cfg, Work& w,
                                       int& iters, bool active, bool* plain) {
     const int n = c.n, nn = c.num_nodes, lane = threadIdx.x & 31;
@@ -486,14 +504,14 @@ __device__ inline int newton_run_warp(const DevCircuit& c, const SoA& dv, size_t
         if (PREC == SP_PREC_FP64) {
             for (int i = 0; i < n * n; ++i) w.A[i] = 0.0;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            PlainSinkRec k(w.A, w.v, w.x, n, lane);
+            auto k = make_sink<TEAM, PlainSinkRec>(w.team, w.A, w.v, w.x, n, lane);
             stamp_all(c, dv, s, k, STAMP_PLAIN, 0.0);
             __syncwarp();
             ok = lu_solve_warp<double>(n, lane, w.A, w.v, k.rows, plain);
         } else {
             for (int i = 0; i < n * n; ++i) w.J[i] = 0.0f;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            MixedSinkRec k(w.J, w.v, w.x, n, lane);
+            auto k = make_sink<TEAM, MixedSinkRec>(w.team, w.J, w.v, w.x, n, lane);
             stamp_all(c, dv, s, k, STAMP_PLAIN, 0.0);
             __syncwarp();
             for (int i = 0; i < n; ++i) w.d[i] = (float)(-w.v[i]);
@@ -521,10 +539,10 @@ __device__ inline int newton_run_warp(const DevCircuit& c, const SoA& dv, size_t
 }
 
 // max_i<num_nodes |F_i| of the FP64 KCL residual at w.x (uses w.v as scratch).
-template <class DV>
+template <bool TEAM = false, class DV>
 __device__ inline double kcl_residual(const DevCircuit& c, const DV& dv, size_t s, Work& w) {
     for (int i = 0; i < c.n; ++i) w.v[i] = 0.0;
-    ResidSink k{w.v, w.x};
+    auto k = make_sink<TEAM, ResidSink>(w.team, w.v, w.x);
     stamp_all(c, dv, s, k, STAMP_PLAIN, 0.0);
     double r = 0.0;
     for (int i = 0; i < c.num_nodes; ++i) r = fmax(r, fabs(w.v[i]));
@@ -570,6 +588,9 @@ struct NewtonLaunch {
     // params is not read), and what the fallback needs to draw its samples in FP64
     const float* params32 = nullptr;
     RedrawArgs redraw;
+    // lanes per sample (a power of two): the primary kernel's, and the most the
+    // fallback takes where its list leaves lanes idle
+    int team = 1, fallback_team = 1;
     // iteration limit of the specialised kernel's cold restart of a sample
     // whose warm start missed (the full limit; cfg may hold the warm cap)
     int cold_max_iterations = 0;
@@ -603,13 +624,14 @@ namespace SP_KERNEL_NS {
 
 // Phase 1: Newton from the warm start (or the circuit's nodeset, or zero)
 // for every sample; misses go to the fallback list.
-template <int PREC>
+template <int PREC, bool TEAM = false>
 __global__ void newton_primary_kernel(NewtonLaunch L) {
     extern __shared__ __align__(16) unsigned char smem[];
     pdl_wait();
     pdl_trigger();
-    const uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t s = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / (TEAM ? (unsigned)L.team : 1u);
     Work w = make_work<PREC>(smem, L.c.n, blockDim.x, threadIdx.x);
+    w.team = TEAM ? L.team : 1;
     const int n = L.c.n;
     const bool warm = L.x0 != nullptr;
     int it = 0, code;
@@ -617,7 +639,7 @@ __global__ void newton_primary_kernel(NewtonLaunch L) {
     // a skipped product with a zero could leave a -0 where the reference has +0
     if (s >= L.count) return;
     load_start(L, s, w, warm);
-    code = newton_run<PREC>(L.c, L.dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
+    code = newton_run<PREC, TEAM>(L.c, L.dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
 #else
     const bool active = s < L.count;
     const uint64_t sd = active ? s : L.count - 1;
@@ -626,25 +648,30 @@ __global__ void newton_primary_kernel(NewtonLaunch L) {
         asm volatile("prefetch.global.L1 [%0];" ::"l"(L.dv.p + (size_t)k * L.dv.stride + sd));
     bool plain = true;
     load_start(L, sd, w, warm);
-    code = newton_run_warp<PREC>(L.c, L.dv, sd, L.cfg, w, it, active, &plain);
+    code = newton_run_warp<PREC, TEAM>(L.c, L.dv, sd, L.cfg, w, it, active, &plain);
     if (!active) return;
     if (!plain) {
         load_start(L, s, w, warm);
-        code = newton_run<PREC>(L.c, L.dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
+        code = newton_run<PREC, TEAM>(L.c, L.dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
     }
 #endif
+    const bool lead = !TEAM || (threadIdx.x & (L.team - 1)) == 0;  // the others hold the same values
     uint8_t st = finish_status(code, w, n) | (warm ? SP_ST_FLAG_WARM : 0);
-    for (int i = 0; i < n; ++i) L.x[s * n + i] = w.x[i];
-    if (L.iters) L.iters[s] = it;
+    if (lead)
+        for (int i = 0; i < n; ++i) L.x[s * n + i] = w.x[i];
+    if (lead && L.iters) L.iters[s] = it;
     bool need_fallback = (st & SP_ST_MASK) != SP_ST_CONVERGED &&
                          (warm || (L.cfg.fallback & (SP_FALLBACK_GMIN | SP_FALLBACK_SOURCE)));
     if (need_fallback) {
-        unsigned int slot = atomicAdd(L.fail_count, 1u);
-        L.fail_list[slot] = (uint32_t)s;
+        if (lead) {
+            unsigned int slot = atomicAdd(L.fail_count, 1u);
+            L.fail_list[slot] = (uint32_t)s;
+        }
     } else if (L.resid) {
-        L.resid[s] = kcl_residual(L.c, L.dv, s, w);
+        const double r = kcl_residual<TEAM>(L.c, L.dv, s, w);
+        if (lead) L.resid[s] = r;
     }
-    if (L.status) L.status[s] = st;
+    if (lead && L.status) L.status[s] = st;
 }
 
 }  // namespace SP_KERNEL_NS
@@ -653,7 +680,7 @@ __global__ void newton_primary_kernel(NewtonLaunch L) {
 // output row (global), the trial iterate in shared memory.  A failed attempt
 // is repeated by the reference with the identical initial guess and stamper,
 // so its outcome repeats; those repeats are accounted without recomputation.
-template <int PREC, class DV>
+template <int PREC, bool TEAM, class DV>
 __device__ inline int gmin_stepping(const NewtonLaunch& L, const DV& dv, size_t s, Work& w, int& total) {
     const int n = L.c.n;
     const sp_newton_config& cfg = L.cfg;
@@ -665,7 +692,7 @@ __device__ inline int gmin_stepping(const NewtonLaunch& L, const DV& dv, size_t 
         ++levels;
         for (int i = 0; i < n; ++i) w.x[i] = sol[i];
         int it = 0;
-        int code = newton_run<PREC>(L.c, dv, s, cfg, STAMP_GMIN, g, w, it);
+        int code = newton_run<PREC, TEAM>(L.c, dv, s, cfg, STAMP_GMIN, g, w, it);
         total += it;
         if (code == NR_SINGULAR) return NR_SINGULAR;
         if (code != NR_CONVERGED) {
@@ -681,7 +708,7 @@ __device__ inline int gmin_stepping(const NewtonLaunch& L, const DV& dv, size_t 
 }
 
 // source stepping (newton.rs:261-356).
-template <int PREC, class DV>
+template <int PREC, bool TEAM, class DV>
 __device__ inline int source_stepping(const NewtonLaunch& L, const DV& dv, size_t s, Work& w, int& total) {
     const int n = L.c.n;
     const sp_newton_config& cfg = L.cfg;
@@ -695,7 +722,7 @@ __device__ inline int source_stepping(const NewtonLaunch& L, const DV& dv, size_
         double cur = fmin(factor, 1.0);
         for (int i = 0; i < n; ++i) w.x[i] = sol[i];
         int it = 0;
-        int code = newton_run<PREC>(L.c, dv, s, cfg, STAMP_SCALED, cur, w, it);
+        int code = newton_run<PREC, TEAM>(L.c, dv, s, cfg, STAMP_SCALED, cur, w, it);
         total += it;
         if (code == NR_SINGULAR) return NR_SINGULAR;
         if (code != NR_CONVERGED) {
@@ -719,7 +746,7 @@ namespace SP_KERNEL_NS {
 
 // Phase 2: the fallback chain for the samples phase 1 missed (grid-stride
 // over the miss list, whose length is only known on the device).
-template <int PREC>
+template <int PREC, bool TEAM = false>
 __global__ void newton_fallback_kernel(NewtonLaunch L) {
     extern __shared__ __align__(16) unsigned char smem[];
     pdl_wait();
@@ -729,9 +756,15 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
     const bool warm = L.x0 != nullptr || L.lin != nullptr;  // listed samples started warm
     const unsigned int misses = *L.fail_count;
     const SoACg dv{L.dv.p, L.dv.stride};
+    // A short list leaves most lanes idle: each sample then has a team of lanes
+    // (with its data in every lane, written alike by all of them).
+    const unsigned team = TEAM && (uint64_t)misses * L.fallback_team <= (uint64_t)gridDim.x * blockDim.x ? L.fallback_team : 1;
+    const unsigned mates = (team == 32 ? 0xffffffffu : (1u << team) - 1u) << (threadIdx.x & 31 & -team);
+    const bool lead = !TEAM || (threadIdx.x & (team - 1)) == 0;
+    w.team = (int)team;
     // neighbours in the list go to different blocks: chains differ in length at
     // every level, and lanes of one warp wait for each other there
-    for (unsigned int j = threadIdx.x * gridDim.x + blockIdx.x; j < misses; j += gridDim.x * blockDim.x) {
+    for (unsigned int j = threadIdx.x / team * gridDim.x + blockIdx.x; j < misses; j += gridDim.x * (blockDim.x / team)) {
         const size_t s = L.fail_list[j];
         if (L.redraw.derived) redraw_sample(L.c, L.redraw, L.dv.stride, s);
         int total = L.iters ? L.iters[s] : 0;
@@ -748,28 +781,30 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
         // the specialised kernel has already restarted this sample cold (status
         // flag), so the chain continues with gmin stepping
         const bool cold_done = warm && L.status && (L.status[s] & SP_ST_FLAG_COLD);
+        if (TEAM) __syncwarp(mates);  // read before the leader writes them
         if (cold_done) flags |= SP_ST_FLAG_COLD;
         if (warm && !cold_done) {
             flags |= SP_ST_FLAG_COLD;
             load_start(L, s, w, false);
             int it = 0;
-            code = newton_run<PREC>(L.c, dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
+            code = newton_run<PREC, TEAM>(L.c, dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
             total += it;
             for (int i = 0; i < n; ++i) L.x[s * n + i] = w.x[i];
         }
         if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_GMIN)) {
             flags |= SP_ST_FLAG_GMIN;
-            code = gmin_stepping<PREC>(L, dv, s, w, total);
+            code = gmin_stepping<PREC, TEAM>(L, dv, s, w, total);
         }
         if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_SOURCE)) {
             flags |= SP_ST_FLAG_SOURCE;
-            code = source_stepping<PREC>(L, dv, s, w, total);
+            code = source_stepping<PREC, TEAM>(L, dv, s, w, total);
         }
         for (int i = 0; i < n; ++i) w.x[i] = L.x[s * n + i];
         uint8_t st = finish_status(code, w, n) | flags;
-        if (L.iters) L.iters[s] = total;
-        if (L.status) L.status[s] = st;
-        if (L.resid) L.resid[s] = kcl_residual(L.c, dv, s, w);
+        const double res = L.resid ? kcl_residual<TEAM>(L.c, dv, s, w) : 0.0;
+        if (lead && L.iters) L.iters[s] = total;
+        if (lead && L.status) L.status[s] = st;
+        if (lead && L.resid) L.resid[s] = res;
     }
 }
 
