@@ -20,6 +20,7 @@
 #include "internal.h"
 #include "mlp_act.cuh"
 #include "mlp_tc.h"
+#include "pdl.cuh"
 #include "rng.cuh"
 
 using bf16 = __nv_bfloat16;
@@ -81,6 +82,8 @@ template <int EPI>
 __global__ void __launch_bounds__(128) gemm_tn(GemmArgs g) {
     __shared__ __align__(16) bf16 sA[2][BM * PITCH];
     __shared__ __align__(16) bf16 sB[2][BN * PITCH];
+    pdl_wait();
+    pdl_trigger();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = warp >> 1, wn = warp & 1;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
@@ -192,55 +195,82 @@ cudaError_t gemm(const GemmArgs& g, int splits, cudaStream_t st) {
         if (mlptc::gemm_supported(t)) return mlptc::gemm(t, splits, st);
     }
     dim3 grid((g.M + BM - 1) / BM, (g.N + BN - 1) / BN, splits);
-    gemm_tn<EPI><<<grid, 128, 0, st>>>(g);
-    return cudaGetLastError();
+    return launch_chained(gemm_tn<EPI>, grid, dim3(128), 0, st, g);
 }
 
-// Sum split-K partials in split order: out[m][n] = sum_z part[z][m][n].
-__global__ void splitk_reduce(const float* __restrict__ part, int splits, int count, float* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float s = 0.f;
-    for (int z = 0; z < splits; ++z) s += part[(size_t)z * count + i];
-    out[i] = s;
-}
-
-// Bias gradient: db[n] = sum over rows of dZ[row][n], in a fixed order: block
-// (x, y) sums rows [y chunk, (y + 1) chunk) of columns 32x.. into part[y][n]
-// (eight row lanes, then the lanes in order); bias_grad_final adds the
-// chunks in order.  kBiasChunks chunks keep the whole GPU busy.
+// The two reductions of a layer's gradients in one launch, each in a fixed order.
+//  * dW: the split-K partials in split order, out[i] = sum_z part[z][i];
+//  * db[n] = sum over rows of dZ[row][n]: block (x, y) behind the first
+//    `wblocks` sums rows [y chunk, (y + 1) chunk) of columns 32x.. into
+//    bpart[y][n] (eight row lanes, then the lanes in order); bias_grad_final
+//    adds the chunks in order, for all layers at once.  kBiasChunks chunks keep
+//    the whole GPU busy.
+// These kernels move a few MB; what they cost is launches: two fewer per layer,
+// and every kernel of the step placed while its predecessor drains, took the
+// gradient step of 17 -> 3 x 256 -> 12 on 4,096 rows from 183 to 124 us (26
+// launches to 18).
 constexpr int kBiasChunks = 64;
 
-__global__ void bias_grad(const bf16* __restrict__ d, int rows, int cols, int ld, float* __restrict__ part) {
+struct ReduceArgs {
+    const float* part;
+    float* out;
+    const bf16* d;
+    float* bpart;
+    int splits, count, wblocks, rows, cols, xblocks, chunks;
+};
+
+__global__ void reduce_grads(ReduceArgs a) {
     __shared__ float sh[8][33];
+    pdl_wait();
+    pdl_trigger();
+    if ((int)blockIdx.x < a.wblocks) {
+        const int i = blockIdx.x * blockDim.x + threadIdx.x;
+        if (i >= a.count) return;
+        float s = 0.f;
+        for (int z = 0; z < a.splits; ++z) s += a.part[(size_t)z * a.count + i];
+        a.out[i] = s;
+        return;
+    }
+    const int bx = (blockIdx.x - a.wblocks) % a.xblocks, by = (blockIdx.x - a.wblocks) / a.xblocks;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int col = blockIdx.x * 32 + tx;
-    const int chunk = (rows + gridDim.y - 1) / gridDim.y;
-    const int r0 = blockIdx.y * chunk, r1 = min(rows, r0 + chunk);
+    const int col = bx * 32 + tx;
+    const int chunk = (a.rows + a.chunks - 1) / a.chunks;
+    const int r0 = by * chunk, r1 = min(a.rows, r0 + chunk);
     float s = 0.f;
-    if (col < cols)
-        for (int r = r0 + ty; r < r1; r += 8) s += __bfloat162float(d[(size_t)r * ld + col]);
+    if (col < a.cols)
+        for (int r = r0 + ty; r < r1; r += 8) s += __bfloat162float(a.d[(size_t)r * a.cols + col]);
     sh[ty][tx] = s;
     __syncthreads();
-    if (ty == 0 && col < cols) {
+    if (ty == 0 && col < a.cols) {
         float t = 0.f;
         for (int k = 0; k < 8; ++k) t += sh[k][tx];
-        part[(size_t)blockIdx.y * cols + col] = t;
+        a.bpart[(size_t)by * a.cols + col] = t;
     }
 }
 
-__global__ void bias_grad_final(const float* __restrict__ part, int chunks, int cols, float* __restrict__ db) {
-    const int col = blockIdx.x * blockDim.x + threadIdx.x;
+constexpr int kBiasLayers = 8;  // layers of one bias_grad_final launch
+struct BiasFinalArgs {
+    const float* part[kBiasLayers];
+    float* db[kBiasLayers];
+    int cols[kBiasLayers], chunks[kBiasLayers];
+};
+
+__global__ void bias_grad_final(BiasFinalArgs a) {
+    pdl_wait();
+    pdl_trigger();
+    const int l = blockIdx.y, col = blockIdx.x * blockDim.x + threadIdx.x, cols = a.cols[l];
     if (col >= cols) return;
     float t = 0.f;
-    for (int y = 0; y < chunks; ++y) t += part[(size_t)y * cols + col];
-    db[col] = t;
+    for (int y = 0; y < a.chunks[l]; ++y) t += a.part[l][(size_t)y * cols + col];
+    a.db[l][col] = t;
 }
 
 // Mean-squared-error gradient of the output layer (first n_real columns),
 // written as dY [rows][ldy] and dY^T [ldy][rows]; accumulates the loss.
 __global__ void mse_grad(const float* __restrict__ y, const float* __restrict__ t, int rows, int n_real, int ldy,
                          int ldt_in, bf16* __restrict__ dy, bf16* __restrict__ dyt, float* __restrict__ loss) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float l = 0.f;
     if (i < rows * ldy) {
@@ -277,6 +307,8 @@ struct AdamArgs {
 };
 
 __global__ void adam(AdamArgs a) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.count) return;
     const int t = *a.step + 1;
@@ -298,7 +330,11 @@ __global__ void adam(AdamArgs a) {
     }
 }
 
-__global__ void bump(int* step) { *step += 1; }
+__global__ void bump(int* step) {
+    pdl_wait();
+    pdl_trigger();
+    *step += 1;
+}
 
 // BF16 copies of one weight tensor (after init or a host upload).
 __global__ void refresh_bf16(const float* w, int rows, int cols, bf16* wt_bf, bf16* w_bf) {
@@ -313,6 +349,8 @@ __global__ void refresh_bf16(const float* w, int rows, int cols, bf16* wt_bf, bf
 // zero in the padding.
 __global__ void pack_inputs(const float* __restrict__ x, int rows, int rows_pad, int n_in, int kin,
                             bf16* __restrict__ X, bf16* __restrict__ Xt) {
+    pdl_wait();
+    pdl_trigger();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows_pad * kin) return;
     const int r = i / kin, c = i % kin;
@@ -554,6 +592,7 @@ struct sp_mlp {
     float* Y = nullptr;
     bf16 *dY = nullptr, *dYt = nullptr, *dA = nullptr, *dB = nullptr, *dAt = nullptr, *dBt = nullptr;
     float* part = nullptr;  // split-K partials
+    float* bias_part = nullptr;  // [layer][kBiasChunks][width] partial bias gradients
     size_t part_elems = 0;
     float* loss = nullptr;
 };
@@ -597,6 +636,7 @@ int ensure_ws(sp_mlp* m, int rows) {
     const int splits = (rp + kSplitRows - 1) / kSplitRows;
     size_t maxw = (size_t)Hd * std::max(Hd, std::max(m->kin, m->kout));
     size_t opart = take(4ull * splits * maxw);
+    size_t obias = take(4ull * m->L * kBiasChunks * std::max(Hd, m->kout));
     size_t oloss = take(256);
     // the callers hold the context's ordering guard: the old workspace is
     // freed in stream order after its last user
@@ -626,6 +666,7 @@ int ensure_ws(sp_mlp* m, int rows) {
     m->dBt = (bf16*)(p + odBt);
     m->part = (float*)(p + opart);
     m->part_elems = splits * maxw;
+    m->bias_part = (float*)(p + obias);
     m->loss = (float*)(p + oloss);
     return SP_OK;
 }
@@ -686,15 +727,16 @@ cudaError_t backward(sp_mlp* m, int rows_pad, const float* targets, int ldt_in, 
     cudaError_t e;
     {
         const int total = rows_pad * m->kout;
-        mse_grad<<<(total + 255) / 256, 256, 0, st>>>(m->Y, targets, rows_pad, m->d.n_out, m->kout, ldt_in, m->dY,
-                                                      m->dYt, m->loss);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = launch_chained(mse_grad, dim3((total + 255) / 256), dim3(256), 0, st, m->Y, targets, rows_pad, m->d.n_out,
+                           m->kout, ldt_in, m->dY, m->dYt, m->loss);
+        if (e != cudaSuccess) return e;
     }
     const int splits = (rows_pad + kSplitRows - 1) / kSplitRows;
     const bf16* dcur = m->dY;    // dZ of the current layer [rows][width]
     const bf16* dcurT = m->dYt;  // transposed [width][rows]
     int width = m->kout;
     bool toggle = false;
+    BiasFinalArgs bf{};
     for (int l = nl; l >= 0; --l) {
         const bf16* inT = (l == 0) ? m->Xt : m->Ht[l - 1];
         const int in_w = (l == 0) ? m->kin : m->H;
@@ -712,16 +754,22 @@ cudaError_t backward(sp_mlp* m, int rows_pad, const float* targets, int ldt_in, 
         g.C32 = m->part;
         g.ldc = in_w;
         if ((e = gemm<EPI_F32>(g, splits, st)) != cudaSuccess) return e;
-        const int cnt = width * in_w;
-        splitk_reduce<<<(cnt + 255) / 256, 256, 0, st>>>(m->part, splits, cnt, m->grads + m->woff[l]);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        {
-            const int chunks = (int)std::max<size_t>(
-                1, std::min<size_t>({(size_t)kBiasChunks, (size_t)rows_pad / 64, m->part_elems / (size_t)width}));
-            bias_grad<<<dim3((width + 31) / 32, chunks), 256, 0, st>>>(dcur, rows_pad, width, width, m->part);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
-            bias_grad_final<<<(width + 127) / 128, 128, 0, st>>>(m->part, chunks, width, m->grads + m->boff[l]);
-            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        const int chunks = (int)std::max<size_t>(
+            1, std::min<size_t>({(size_t)kBiasChunks, (size_t)rows_pad / 64, m->part_elems / (size_t)width}));
+        ReduceArgs ra{m->part, m->grads + m->woff[l], dcur,
+                      m->bias_part + (size_t)l * kBiasChunks * std::max(m->H, m->kout),
+                      splits, width * in_w, (width * in_w + 255) / 256, rows_pad, width, (width + 31) / 32, chunks};
+        e = launch_chained(reduce_grads, dim3(ra.wblocks + ra.xblocks * chunks), dim3(256), 0, st, ra);
+        if (e != cudaSuccess) return e;
+        bf.part[l % kBiasLayers] = ra.bpart;
+        bf.db[l % kBiasLayers] = m->grads + m->boff[l];
+        bf.cols[l % kBiasLayers] = width;
+        bf.chunks[l % kBiasLayers] = chunks;
+        if (l % kBiasLayers == 0) {  // the layers from here up to the last multiple
+            const int count = std::min(nl + 1 - l, kBiasLayers);
+            const dim3 grid((std::max(m->H, m->kout) + 127) / 128, count);
+            e = launch_chained(bias_grad_final, grid, dim3(128), 0, st, bf);
+            if (e != cudaSuccess) return e;
         }
         if (l == 0) break;
         // input gradient through the GELU: dZ_{l-1} = (dZ_l * W_l) .* gelu'(Z_{l-1})
@@ -770,7 +818,8 @@ cudaError_t adam_step(sp_mlp* m, float lr, int total_steps, cudaStream_t st) {
         a.cols = m->cols[l];
         a.wt_bf = m->wt_bf + m->woff[l];
         a.w_bf = m->w_bf + m->woff[l];
-        adam<<<(a.count + 255) / 256, 256, 0, st>>>(a);
+        cudaError_t e = launch_chained(adam, dim3((a.count + 255) / 256), dim3(256), 0, st, a);
+        if (e != cudaSuccess) return e;
         AdamArgs b = a;
         b.w = m->params + m->boff[l];
         b.m = m->adam_m + m->boff[l];
@@ -778,10 +827,10 @@ cudaError_t adam_step(sp_mlp* m, float lr, int total_steps, cudaStream_t st) {
         b.g = m->grads + m->boff[l];
         b.count = m->rows[l];
         b.rows = 0;
-        adam<<<(b.count + 255) / 256, 256, 0, st>>>(b);
+        e = launch_chained(adam, dim3((b.count + 255) / 256), dim3(256), 0, st, b);
+        if (e != cudaSuccess) return e;
     }
-    bump<<<1, 1, 0, st>>>(m->step);
-    return cudaGetLastError();
+    return launch_chained(bump, dim3(1), dim3(1), 0, st, m->step);
 }
 
 cudaError_t refresh_all(sp_mlp* m, cudaStream_t st) {
@@ -959,8 +1008,10 @@ int sp_mlp_gradients_device(sp_mlp* m, const float* d_x, const float* d_t, uint6
     ScratchOrder order(m->ctx, st);  // orders workspace reuse and growth after earlier users
     if (ensure_ws(m, (int)rows) != SP_OK) return mlp_fail(m->ctx, SP_ERR_MEMORY_ALLOC, "MLP workspace");
     const int rp = (int)rows;
-    pack_inputs<<<(rp * m->kin + 255) / 256, 256, 0, st>>>(d_x, rp, rp, m->d.n_in, m->kin, m->X, m->Xt);
     cudaMemsetAsync(m->loss, 0, 4, st);
+    if (launch_chained(pack_inputs, dim3((rp * m->kin + 255) / 256), dim3(256), 0, st, d_x, rp, rp, m->d.n_in, m->kin,
+                       m->X, m->Xt) != cudaSuccess)
+        return mlp_fail(m->ctx, SP_ERR_BACKEND, "MLP gradients");
     if (forward(m, rp, true, st) != cudaSuccess || backward(m, rp, d_t, m->d.n_out, st) != cudaSuccess)
         return mlp_fail(m->ctx, SP_ERR_BACKEND, "MLP gradients");
     cudaMemcpyAsync(d_grads, m->grads, m->nparams * 4, cudaMemcpyDeviceToDevice, st);
@@ -987,8 +1038,9 @@ int sp_mlp_train_device(sp_mlp* m, const float* d_x, const float* d_t, uint64_t 
         for (uint64_t s = 0; s < steps_per_epoch; ++s) {
             const float* xb = d_x + s * batch * m->d.n_in;
             const float* tb = d_t + s * batch * m->d.n_out;
-            pack_inputs<<<(batch * m->kin + 255) / 256, 256, 0, st>>>(xb, batch, batch, m->d.n_in, m->kin, m->X,
-                                                                      m->Xt);
+            if (launch_chained(pack_inputs, dim3((batch * m->kin + 255) / 256), dim3(256), 0, st, xb, batch, batch,
+                               m->d.n_in, m->kin, m->X, m->Xt) != cudaSuccess)
+                return mlp_fail(m->ctx, SP_ERR_BACKEND, "MLP training step");
             if (forward(m, batch, true, st) != cudaSuccess || backward(m, batch, tb, m->d.n_out, st) != cudaSuccess ||
                 adam_step(m, lr, total, st) != cudaSuccess)
                 return mlp_fail(m->ctx, SP_ERR_BACKEND, "MLP training step");

@@ -815,6 +815,8 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, 
 template <int EPI>
 __global__ void __launch_bounds__(kGThreads) gemm_kernel(GemmTcArgs g) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
+    pdl_wait();  // before tensor memory is taken: a waiting block holds none
+    pdl_trigger();
     unsigned char* sm = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
     const int bn = g.bn;
     const uint32_t stage_bytes = gemm_stage_bytes(bn);
@@ -1095,13 +1097,11 @@ cudaError_t gemm(GemmTcArgs g, int splits, cudaStream_t st) {
     g.bn = bn;
     const uint32_t smem = gemm_smem_bytes(g.bn);
     const dim3 grid((unsigned)((g.M + 127) / 128), (unsigned)((g.N + g.bn - 1) / g.bn), (unsigned)splits);
-    switch (g.epi) {
-        case kEpiF32: gemm_kernel<kEpiF32><<<grid, kGThreads, smem, st>>>(g); break;
-        case kEpiBiasF32: gemm_kernel<kEpiBiasF32><<<grid, kGThreads, smem, st>>>(g); break;
-        case kEpiBiasGelu: gemm_kernel<kEpiBiasGelu><<<grid, kGThreads, smem, st>>>(g); break;
-        default: gemm_kernel<kEpiGeluBwd><<<grid, kGThreads, smem, st>>>(g); break;
-    }
-    return cudaGetLastError();
+    void (*const kernel)(GemmTcArgs) = g.epi == kEpiF32       ? gemm_kernel<kEpiF32>
+                                       : g.epi == kEpiBiasF32  ? gemm_kernel<kEpiBiasF32>
+                                       : g.epi == kEpiBiasGelu ? gemm_kernel<kEpiBiasGelu>
+                                                               : gemm_kernel<kEpiGeluBwd>;
+    return launch_chained(kernel, grid, dim3(kGThreads), smem, st, g);
 }
 
 }  // namespace mlptc

@@ -1,5 +1,6 @@
 // Programmatic dependent launch for the kernels of one sweep (draw ->
-// warm start -> primary Newton -> fallback -> moments): each is launched
+// warm start -> primary Newton -> fallback -> moments) and of a training step:
+// each is launched
 // with programmatic stream serialisation, so its blocks are placed while its
 // predecessor drains.  Every such kernel starts with pdl_wait()
 // (griddepcontrol.wait: returns once the predecessor grid has completed and
