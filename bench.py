@@ -882,6 +882,16 @@ def main():
                              "roofline": {"bound": "hbm", "achieved": a, "peak": hbm_peak, "unit": "GB/s",
                                           "frac": a / hbm_peak, "bytes": by,
                                           "per_unit": f"{per_it} B per GMRES iteration and corner"}}
+            if prec == abi.SP_PREC_MIXED:
+                # the mixed kernel keeps the basis on chip, so the bytes above are
+                # not HBM traffic: FP32 operations instead (two projections and two
+                # subtractions of k+1 vectors, the stencil)
+                fl = kry * (4 * 2 * 16 + 10) * nG
+                a = fl / (ms * 1e-3) / 1e12
+                fp32_peak = pipe.get("fp32_tflops") or 73.0
+                config5[name]["roofline"] = {"bound": "latency (FP32 operations counted)", "achieved": a,
+                                             "peak": fp32_peak, "unit": "TFLOP/s", "frac": a / fp32_peak, "flops": fl,
+                                             "per_unit": f"{138 * nG} FP32 flops per GMRES iteration and corner"}
         sample5 = 4
         t0 = time.perf_counter()
         oracle.grid_solve(abi.grid_config(), SEED, sample5)

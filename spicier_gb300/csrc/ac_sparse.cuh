@@ -26,7 +26,7 @@
 //
 // Bound: the FP64 pipe (64 cycles per warp instruction of an SM quarter) and,
 // with two warps per quarter, the chains between its instructions.  Op-amp,
-// 8,192 samples x 81 frequencies: 19.5 -> 2.8 ms.
+// 8,192 samples x 81 frequencies: 19.5 -> 2.8 ms (the call with its DC points: 20.0 -> 3.2).
 #pragma once
 #include "ac.cuh"
 

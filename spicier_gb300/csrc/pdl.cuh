@@ -1,8 +1,7 @@
 // Programmatic dependent launch for the kernels of one sweep (draw ->
 // warm start -> primary Newton -> fallback -> moments) and of a training step:
-// each is launched
-// with programmatic stream serialisation, so its blocks are placed while its
-// predecessor drains.  Every such kernel starts with pdl_wait()
+// each is launched with programmatic stream serialisation, so its blocks are
+// placed while its predecessor drains.  Every such kernel starts with pdl_wait()
 // (griddepcontrol.wait: returns once the predecessor grid has completed and
 // its memory is visible) before it touches global memory, then calls
 // pdl_trigger() (griddepcontrol.launch_dependents) so that its own

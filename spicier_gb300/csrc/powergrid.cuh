@@ -6,12 +6,14 @@
 // right-preconditioned GMRES(m) with Givens rotations; the Arnoldi vectors
 // are orthogonalised by classical Gram-Schmidt applied twice (the oracle and
 // the reference use modified Gram-Schmidt: same iterates in exact
-// arithmetic, two block reductions per step instead of k + 1).  Layout: thread t of the CTA owns rows t, t + T, t + 2T, ... of
-// every vector (coalesced), the edge conductances and the Krylov basis live
-// in the instance's global workspace (the basis does not fit on chip), the
-// vector being multiplied lives in shared memory for the stencil's
-// neighbour reads, and every dot product is a fixed-order block reduction
-// (so a run is reproducible; the oracle's sequential sums round differently).
+// arithmetic, two block reductions per step instead of k + 1).  Layout of the
+// FP64 kernel: thread t of the CTA owns rows t, t + T, t + 2T, ... of every
+// vector (coalesced), the edge conductances and the Krylov basis live in the
+// instance's global workspace (an FP64 basis does not fit on chip; for the FP32
+// one see powergrid_mixed.cuh), the vector being multiplied lives in shared
+// memory for the stencil's neighbour reads, and every dot product is a
+// fixed-order block reduction (so a run is reproducible; the oracle's
+// sequential sums round differently).
 //
 //   SP_PREC_FP64   the oracle's algorithm in FP64 (GMRES on A x_new = b);
 //   SP_PREC_MIXED  FP32 Krylov: each Newton iteration solves A d = b - A x
