@@ -85,16 +85,22 @@ __host__ __device__ inline double limit_voltage(double vd, double nvt, double vc
 }
 
 #if defined(__CUDACC__)
-// a < b for finite a, b from their bit patterns (the integer pipe); -0 counts as below +0
+// a < b from their bit patterns (the integer pipe) for a that is a number; -0
+// counts as below +0.  False where b is NaN: one without a sign, which the
+// patterns order above every number, is tested for; one with a sign lies below
+// them all.
 __device__ __forceinline__ bool below_int(double a, double b) {
     const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-    return (x ^ (long long)((unsigned long long)(x >> 63) >> 1)) < (y ^ (long long)((unsigned long long)(y >> 63) >> 1));
+    return (x ^ (long long)((unsigned long long)(x >> 63) >> 1)) < (y ^ (long long)((unsigned long long)(y >> 63) >> 1)) &&
+           y <= 0x7ff0000000000000LL;
 }
 #endif
 
 // Level-1 evaluate (level1.rs:154-191); vth = |VTO|, beta = KP*NF*W/L.
-// INT_TESTS: the region tests as integer comparisons, for finite voltages (a
-// comparison is an FP64-pipe instruction; a zero's sign does not change the result).
+// INT_TESTS: the region tests as integer comparisons, for finite voltages and any
+// parameters (a comparison is an FP64-pipe instruction; a zero's sign does not
+// change the result, and a NaN threshold is in no region but the last, as in
+// floating point).
 template <bool INT_TESTS = false>
 __host__ __device__ inline void mos_eval(bool pmos, double vth, double beta, double lambda, double vgs,
                                 double vds, double& ids, double& gds, double& gm) {
