@@ -378,6 +378,22 @@ __device__ inline bool lu_solve_warp(int n, int lane, Il<T> A, Il<T> b, unsigned
     return ok;
 }
 
+// The lanes that hold a sample together with this one (a power of two of them).
+__device__ __forceinline__ unsigned team_lanes(unsigned team) {
+    return (team == 32 ? 0xffffffffu : (1u << team) - 1u) << (threadIdx.x & 31 & -team);
+}
+// Between a team's accesses to its sample's row in global memory: the leader
+// writes, every lane reads, and each waits for the others in between (a shuffle
+// does not order memory).
+template <bool TEAM>
+__device__ __forceinline__ void team_sync(unsigned team) {
+    if (TEAM) __syncwarp(team_lanes(team));
+}
+template <bool TEAM>
+__device__ __forceinline__ bool team_leads(unsigned team) {
+    return !TEAM || (threadIdx.x & (team - 1)) == 0;
+}
+
 // Shared-memory work area of one thread.
 struct Work {
     Il<double> x;   // current iterate [n]
@@ -676,6 +692,16 @@ __global__ void newton_primary_kernel(NewtonLaunch L) {
 
 }  // namespace SP_KERNEL_NS
 
+// A sample's row of unknowns, written by its team's leader once every lane has
+// read what was there, and there for every lane on return.
+template <bool TEAM, class F>
+__device__ __forceinline__ void put_row(unsigned team, int n, double* row, F value) {
+    team_sync<TEAM>(team);
+    if (team_leads<TEAM>(team))
+        for (int i = 0; i < n; ++i) row[i] = value(i);
+    team_sync<TEAM>(team);
+}
+
 // gmin stepping (newton.rs:373-459).  The level solution lives in the
 // output row (global), the trial iterate in shared memory.  A failed attempt
 // is repeated by the reference with the identical initial guess and stamper,
@@ -685,7 +711,7 @@ __device__ inline int gmin_stepping(const NewtonLaunch& L, const DV& dv, size_t 
     const int n = L.c.n;
     const sp_newton_config& cfg = L.cfg;
     double* sol = L.x + s * n;
-    for (int i = 0; i < n; ++i) sol[i] = 0.0;
+    put_row<TEAM>(w.team, n, sol, [](int) { return 0.0; });
     double g = cfg.gmin_initial;
     int levels = 0;
     while (g >= cfg.gmin_final * 0.99 && levels < 4096) {
@@ -699,7 +725,7 @@ __device__ inline int gmin_stepping(const NewtonLaunch& L, const DV& dv, size_t 
             total += (cfg.gmin_max_attempts - 1) * it;
             return NR_MAXITER;
         }
-        for (int i = 0; i < n; ++i) sol[i] = w.x[i];
+        put_row<TEAM>(w.team, n, sol, [&](int i) { return w.x[i]; });
         if (g <= cfg.gmin_final) break;
         g /= cfg.gmin_reduction;
         if (g < cfg.gmin_final) g = cfg.gmin_final;
@@ -713,7 +739,7 @@ __device__ inline int source_stepping(const NewtonLaunch& L, const DV& dv, size_
     const int n = L.c.n;
     const sp_newton_config& cfg = L.cfg;
     double* sol = L.x + s * n;
-    for (int i = 0; i < n; ++i) sol[i] = 0.0;
+    put_row<TEAM>(w.team, n, sol, [](int) { return 0.0; });
     double factor = cfg.src_initial;
     double step = cfg.src_step;
     int guard = 0;
@@ -734,7 +760,7 @@ __device__ inline int source_stepping(const NewtonLaunch& L, const DV& dv, size_
             }
             return NR_MAXITER;
         }
-        for (int i = 0; i < n; ++i) sol[i] = w.x[i];
+        put_row<TEAM>(w.team, n, sol, [&](int i) { return w.x[i]; });
         if (fabs(cur - 1.0) < 1e-9) break;
         factor += step;
         if (step < cfg.src_step) step = fmin(step * 1.5, cfg.src_step);
@@ -756,11 +782,12 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
     const bool warm = L.x0 != nullptr || L.lin != nullptr;  // listed samples started warm
     const unsigned int misses = *L.fail_count;
     const SoACg dv{L.dv.p, L.dv.stride};
-    // A short list leaves most lanes idle: each sample then has a team of lanes
-    // (with its data in every lane, written alike by all of them).
+    // A short list leaves most lanes idle: each sample then has a team of lanes,
+    // every one of them with its data.  All of them take the same branches: what
+    // decides one comes from values that each has computed alike, or from the
+    // sample's row, which changes only in put_row.
     const unsigned team = TEAM && (uint64_t)misses * L.fallback_team <= (uint64_t)gridDim.x * blockDim.x ? L.fallback_team : 1;
-    const unsigned mates = (team == 32 ? 0xffffffffu : (1u << team) - 1u) << (threadIdx.x & 31 & -team);
-    const bool lead = !TEAM || (threadIdx.x & (team - 1)) == 0;
+    const bool lead = team_leads<TEAM>(team);
     w.team = (int)team;
     // neighbours in the list go to different blocks: chains differ in length at
     // every level, and lanes of one warp wait for each other there
@@ -781,7 +808,7 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
         // the specialised kernel has already restarted this sample cold (status
         // flag), so the chain continues with gmin stepping
         const bool cold_done = warm && L.status && (L.status[s] & SP_ST_FLAG_COLD);
-        if (TEAM) __syncwarp(mates);  // read before the leader writes them
+        team_sync<TEAM>(team);  // read before the leader writes them
         if (cold_done) flags |= SP_ST_FLAG_COLD;
         if (warm && !cold_done) {
             flags |= SP_ST_FLAG_COLD;
@@ -789,7 +816,7 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
             int it = 0;
             code = newton_run<PREC, TEAM>(L.c, dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
             total += it;
-            for (int i = 0; i < n; ++i) L.x[s * n + i] = w.x[i];
+            put_row<TEAM>(team, n, L.x + s * n, [&](int i) { return w.x[i]; });
         }
         if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_GMIN)) {
             flags |= SP_ST_FLAG_GMIN;
