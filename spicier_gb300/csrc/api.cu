@@ -462,12 +462,12 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     }
     const size_t bg = align256(sizeof(float4) * gauss.size());
     // the AC matrix's real entries (ac_real_stamps' positions, in order of first
-    // touch) and the elements with imaginary ones
+    // touch) and the elements with imaginary ones; larger circuits have no AC sweep
     std::vector<AcEntry> acent;
     std::vector<AcReact> acreact;
     int acvals = 0;
-    {
-        std::vector<char> seen((size_t)std::max(t->n, 1) * std::max(t->n, 1), 0);
+    if (t->n <= kMaxDenseN) {
+        std::vector<char> seen((size_t)t->n * t->n, 0);
         auto put = [&](int r, int col) {
             if (r < 0 || col < 0 || seen[(size_t)col * t->n + r]) return;
             seen[(size_t)col * t->n + r] = 1;
@@ -475,7 +475,7 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
         };
         auto cond = [&](int i, int j) { put(i, i), put(j, j), put(i, j), put(j, i); };
         auto vccs = [&](int op, int on, int cp, int cn) { put(op, cp), put(op, cn), put(on, cp), put(on, cn); };
-        for (int e = 0; e < c->num_elements && t->n <= 256; ++e) {
+        for (int e = 0; e < c->num_elements; ++e) {
             const sp_element& el = c->elements[e];
             const int a0 = el.node[0], a1 = el.node[1], a2 = el.node[2], a3 = el.node[3], br = c->num_nodes + el.branch;
             switch (el.kind) {
