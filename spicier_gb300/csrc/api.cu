@@ -499,53 +499,52 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
         for (AcReact& r : acreact) r.val += (int)acent.size();
     }
     const size_t bae = align256(sizeof(AcEntry) * acent.size()), bar = align256(sizeof(AcReact) * acreact.size());
-    cudaError_t e = cudaMalloc(&t->dev, be + bp + bu + bo + bn + bw + bt + bg + bae + bar + 256);
+    // every part in one buffer and one copy: a blocking copy costs several
+    // microseconds whatever its size
+    std::vector<char> stage;
+    auto part = [&](size_t bytes, const void* src, size_t used) {
+        const size_t at = stage.size();
+        stage.resize(at + bytes);
+        if (used) std::memcpy(stage.data() + at, src, used);
+        return at;
+    };
+    stage.reserve(be + bp + bu + bo + bn + bw + bt + bg + bae + bar);
+    const size_t oel = part(be, c->elements, sizeof(sp_element) * c->num_elements);
+    const size_t opar = part(bp, c->params, sizeof(sp_param) * c->num_params);
+    const size_t opul = part(bu, c->pulses, sizeof(sp_pulse) * c->num_pulses);
+    const size_t odoff = part(bo, doff.data(), sizeof(int) * doff.size());
+    if (!b3.empty()) std::memcpy(stage.data() + odoff + sizeof(int) * doff.size(), b3.data(), sizeof(int) * b3.size());
+    const size_t ons = part(bn, c->nodeset, c->nodeset ? sizeof(double) * t->n : 0);
+    const size_t odrawn = part(bw, drawn.data(), sizeof(int) * drawn.size());
+    const size_t otran = part(bt, tran.data(), sizeof(TransientEl) * tran.size());
+    const size_t ogauss = part(bg, gauss.data(), sizeof(float4) * gauss.size());
+    const size_t oac = part(bae, acent.data(), sizeof(AcEntry) * acent.size());
+    part(bar, acreact.data(), sizeof(AcReact) * acreact.size());
+    cudaError_t e = cudaMalloc(&t->dev, stage.size() + 256);
     if (e != cudaSuccess) {
         delete t;
         return cuda_fail(ctx, e, "topology allocation");
     }
     char* b = (char*)t->dev;
-    sp_element* del = (sp_element*)b;
-    sp_param* dpar = (sp_param*)(b + be);
-    sp_pulse* dpul = (sp_pulse*)(b + be + bp);
-    int* ddoff = (int*)(b + be + bp + bu);
-    double* dns = (double*)(b + be + bp + bu + bo);
-    int* ddrawn = (int*)(b + be + bp + bu + bo + bn);
-    TransientEl* dtran = (TransientEl*)(b + be + bp + bu + bo + bn + bw);
-    float4* dgauss = (float4*)(b + be + bp + bu + bo + bn + bw + bt);
-    char* dac = b + be + bp + bu + bo + bn + bw + bt + bg;
-    if (!acent.empty()) e = cudaMemcpy(dac, acent.data(), sizeof(AcEntry) * acent.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !acreact.empty())
-        e = cudaMemcpy(dac + bae, acreact.data(), sizeof(AcReact) * acreact.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !gauss.empty()) e = cudaMemcpy(dgauss, gauss.data(), sizeof(float4) * gauss.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !tran.empty()) e = cudaMemcpy(dtran, tran.data(), sizeof(TransientEl) * tran.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && c->num_elements) e = cudaMemcpy(del, c->elements, sizeof(sp_element) * c->num_elements, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !drawn.empty())
-        e = cudaMemcpy(ddrawn, drawn.data(), sizeof(int) * drawn.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && c->num_params)
-        e = cudaMemcpy(dpar, c->params, sizeof(sp_param) * c->num_params, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && c->num_pulses)
-        e = cudaMemcpy(dpul, c->pulses, sizeof(sp_pulse) * c->num_pulses, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && c->num_elements)
-        e = cudaMemcpy(ddoff, doff.data(), sizeof(int) * c->num_elements, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && !b3.empty())
-        e = cudaMemcpy(ddoff + c->num_elements, b3.data(), sizeof(int) * b3.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && c->nodeset) e = cudaMemcpy(dns, c->nodeset, sizeof(double) * t->n, cudaMemcpyHostToDevice);
+    int* ddoff = (int*)(b + odoff);
+    double* dns = (double*)(b + ons);
+    if (!stage.empty()) e = cudaMemcpy(b, stage.data(), stage.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         cudaFree(t->dev);
         delete t;
         return cuda_fail(ctx, e, "topology upload");
     }
     t->dc = DevCircuit{c->num_nodes, c->num_branches, t->n, c->num_elements, c->num_params, nd,
-                       del, dpar, dpul, ddoff, c->nodeset ? dns : nullptr, ddoff + c->num_elements, (int)b3.size()};
-    t->d_tran = dtran;
-    t->d_gauss32 = dgauss;
-    t->d_ac = dac;
+                       (sp_element*)(b + oel), (sp_param*)(b + opar), (sp_pulse*)(b + opul), ddoff,
+                       c->nodeset ? dns : nullptr, ddoff + c->num_elements, (int)b3.size()};
+    t->d_tran = b + otran;
+    t->d_gauss32 = (const float4*)(b + ogauss);
+    t->d_ac = b + oac;
     t->ac_react_off = bae;
     t->num_ac_entries = (int)acent.size();
     t->num_ac_reacts = (int)acreact.size();
     t->num_ac_values = acvals;
-    t->d_drawn = ddrawn;
+    t->d_drawn = (int*)(b + odrawn);
     t->num_drawn = (int)drawn.size();
     t->h_elements.assign(c->elements, c->elements + c->num_elements);
     t->h_params.assign(c->params, c->params + c->num_params);
