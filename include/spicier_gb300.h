@@ -739,9 +739,9 @@ int sp_moments_device(sp_ctx* ctx, const double* d_values, uint64_t rows, uint32
 /* dispatch.rs:85-120).  A setting applies to the sizes of one bucket: key */
 /* "<setting>@<bucket>", bucket = sp_tune_bucket(size) (the smallest power */
 /* of two >= size, at least 4).  Settings and their size:                  */
-/*   lu.cta               1: CTA-per-system batched LU where the rule      */
-/*                        picks one thread per system (FP64 n <= 16,       */
-/*                        mixed n <= 28); size n                           */
+/*   lu.cta               1: CTA-per-system batched LU in FP64 where the   */
+/*                        rule picks one thread per system (n <= 16)       */
+/*   lu.cta.mixed         the same for mixed solves (n <= 28); size n      */
 /*   newton.block.fp64 | .mixed | .exact  threads per block of the generic */
 /*                        thread-per-sample Newton kernels; size MNA n     */
 /*   spec.bpsm.fp64 | .mixed  resident blocks per SM of the topology-      */
@@ -750,7 +750,8 @@ int sp_moments_device(sp_ctx* ctx, const double* d_values, uint64_t rows, uint32
 /*                        (at most what fits); size max_sections           */
 /*   mlp.teams            128-sample tiles in flight per SM of the tcgen05 */
 /*                        warm start (resident weights); size hidden width */
-/* value <= 0 removes a setting.  Results do not depend on any setting.    */
+/* value <= 0 removes a setting.  Results do not depend on any setting but */
+/* lu.cta.mixed: the CTA kernel eliminates in FP64 in every precision.     */
 /* sp_tune_get returns 1 and the value when the key is set, else 0.        */
 /* ---------------------------------------------------------------------- */
 int sp_tune_set(sp_ctx* ctx, const char* key, int value);

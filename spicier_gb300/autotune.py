@@ -8,17 +8,20 @@ built-in heuristics pick threads per instance and tile shapes, and this
 module times the alternatives on the caller's own workload and stores the
 fastest with sp_tune_set (include/spicier_gb300.h lists the settings):
 
-  lu.cta              thread-per-system or CTA-per-system batched LU (n <= 28)
+  lu.cta              thread-per-system or CTA-per-system batched LU, FP64 (n <= 16)
+  lu.cta.mixed        the same for mixed solves (n <= 28)
   newton.block.<p>    threads per block of the thread-per-sample Newton kernels
   spec.bpsm.<p>       resident blocks per SM of the topology-specialised kernel
-  ladder.bpsm         resident blocks per SM of the ladder transients
+  ladder.bpsm         resident blocks per SM of the ladder transients (by default as many as fit)
   mlp.teams           128-sample tiles in flight per SM of the warm-start network
 
-No setting changes any result (each candidate runs the same arithmetic per
-sample); the tuner only times.  A cache file holds, per GPU name, the chosen
-value of every "<setting>@<bucket>" key and the timings that chose it;
-Autotuner.apply() loads it into a context.  A value of 0 stands for the
-built-in heuristic (the key is then absent from the library's table).
+No setting but one changes any result (each candidate runs the same arithmetic
+per sample); the tuner only times.  The exception is lu.cta.mixed, whose CTA
+kernel eliminates in FP64 where the thread kernel refines an FP32 elimination.
+A cache file holds, per GPU name, the chosen value of every
+"<setting>@<bucket>" key and the timings that chose it; Autotuner.apply()
+loads it into a context.  A value of 0 stands for the built-in heuristic (the
+key is then absent from the library's table).
 """
 from __future__ import annotations
 
@@ -135,18 +138,25 @@ class Autotuner:
         return best
 
     # -- the settings ----------------------------------------------------------------
-    def tune_lu(self, sizes=(4, 8, 12, 16, 20, 24, 28), batch: int = 65536) -> Dict[int, int]:
-        """Thread-per-system (0) or CTA-per-system (1) batched LU per size bucket."""
+    def tune_lu(self, sizes=(4, 8, 12, 16, 20, 24, 28), batch: int = 65536,
+                precision: int = abi.SP_PREC_FP64) -> Dict[int, int]:
+        """Thread-per-system (0) or CTA-per-system (1) batched LU per size bucket, timed on
+        solves of `precision`.  FP64 systems of n > 16 have the CTA kernel only (0, not timed)."""
         import torch
         out = {}
         dev = torch.device("cuda", self.ctx.device)
+        mixed = precision == abi.SP_PREC_MIXED
         for n in sizes:
+            if n > 16 and not mixed:
+                out[n] = 0
+                continue
             A = torch.rand((batch, n, n), dtype=torch.float64, device=dev) + n * torch.eye(n, dtype=torch.float64,
                                                                                            device=dev)
             b = torch.rand((batch, n), dtype=torch.float64, device=dev)
             x = torch.empty_like(b)
             sing = torch.empty(batch, dtype=torch.uint8, device=dev)
-            out[n] = self.search("lu.cta", n, (0, 1), lambda: self.ctx.solve_batch_device(A, b, n, batch, x, sing))
+            out[n] = self.search("lu.cta.mixed" if mixed else "lu.cta", n, (0, 1), lambda: self.ctx.solve_batch_device(
+                A, b, n, batch, x, sing, precision=precision))
         return out
 
     def tune_newton(self, topo, precision: int, samples: int = 65536, seed: int = 1) -> Dict[str, int]:
@@ -171,7 +181,7 @@ class Autotuner:
         return out
 
     def tune_ladder(self, cfg, count: int = 1024, seed: int = 1) -> int:
-        """Resident blocks per SM of the ladder transients."""
+        """Resident blocks per SM of the ladder transients: as many as fit (0), or one or two."""
         import torch
         dev = torch.device("cuda", self.ctx.device)
         ld = cfg.max_sections + 2

@@ -291,9 +291,12 @@ static int solve_batch_device_locked(sp_ctx* ctx, const double* d_m, const doubl
     // 11.5 / 3.4: a thread's n^2 doubles of shared memory leave one warp per SM
     // there).  The mixed kernel, half the shared memory, keeps one thread per
     // system up to kMaxDenseN; the tuner may choose the CTA kernel below either
-    // limit (setting "lu.cta", 1 = CTA).
-    const size_t thread_max = precision == SP_PREC_MIXED ? (size_t)kMaxDenseN : 16;
-    const bool cta = n > thread_max || tune_get(ctx, "lu.cta", (long long)n, 0) == 1;
+    // limit (1 = CTA; settings "lu.cta" for FP64 and "lu.cta.mixed", of their own
+    // because they are timed on different kernels and the CTA kernel's mixed
+    // solutions are FP64 ones).
+    const bool mixed = precision == SP_PREC_MIXED;
+    const size_t thread_max = mixed ? (size_t)kMaxDenseN : 16;
+    const bool cta = n > thread_max || tune_get(ctx, mixed ? "lu.cta.mixed" : "lu.cta", (long long)n, 0) == 1;
     if (cta) {
         // one CTA per system, FP64 in the reference's order (both precisions)
         ProfScope prof(ctx, "lu_batch_cta", st);
@@ -310,10 +313,9 @@ static int solve_batch_device_locked(sp_ctx* ctx, const double* d_m, const doubl
         if (e != cudaSuccess) return cuda_fail(ctx, e, "solve_batch launch");
         return SP_OK;
     }
-    ProfScope prof(ctx, precision == SP_PREC_MIXED ? "lu_batch_mixed" : "lu_batch_fp64", st);
-    cudaError_t e = (precision == SP_PREC_MIXED)
-                        ? launch_lu_batch_mixed(d_m, d_r, (int)n, batch, d_x, d_s, refine_steps, st)
-                        : launch_lu_batch_exact(d_m, d_r, (int)n, batch, d_x, d_s, st);
+    ProfScope prof(ctx, mixed ? "lu_batch_mixed" : "lu_batch_fp64", st);
+    cudaError_t e = mixed ? launch_lu_batch_mixed(d_m, d_r, (int)n, batch, d_x, d_s, refine_steps, st)
+                          : launch_lu_batch_exact(d_m, d_r, (int)n, batch, d_x, d_s, st);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "solve_batch launch");
     return SP_OK;
 }
