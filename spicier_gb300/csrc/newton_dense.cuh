@@ -244,6 +244,11 @@ __device__ inline bool lu_solve_fp32(int n, Il<float> A, Il<float> b) {
     return true;
 }
 
+// 2^-500 <= |x| < 2^500
+__device__ __forceinline__ bool mid_range(double x) {
+    return (((unsigned)(__double_as_longlong(x) >> 32) & 0x7fffffffu) >> 20) - 523u < 1000u;
+}
+
 // a / b as IEEE division gives it, given r = 1 / b: two correction steps of the
 // fused remainder (Markstein: r correctly rounded makes the second one round
 // a / b correctly), five FP64 instructions instead of a division's ten, where
@@ -252,10 +257,7 @@ __device__ __forceinline__ double warp_div(double a, double b, double r) {
     const double q0 = a * r;
     double q = fma(fma(-b, q0, a), r, q0);
     q = fma(fma(-b, q, a), r, q);
-    auto middle = [](double x) {  // 2^-500 <= |x| < 2^500
-        return (((unsigned)(__double_as_longlong(x) >> 32) & 0x7fffffffu) >> 20) - 523u < 1000u;
-    };
-    if (!(middle(a) && middle(b))) q = __double_as_longlong(a) << 1 == 0 && middle(b) ? q0 : a / b;
+    if (!(mid_range(a) && mid_range(b))) q = __double_as_longlong(a) << 1 == 0 && mid_range(b) ? q0 : a / b;
     return q;
 }
 __device__ __forceinline__ float warp_div(float a, float b, float) { return a / b; }

@@ -202,8 +202,7 @@ __global__ void transient_fixed_kernel(TransientLaunch L) {
                 at[q][(int)b[i]] = i;
                 const double d = M[i * nt + i];
                 if (d == 0.0) status = SP_ST_SINGULAR;
-                // kept only where the correction step below holds with room to spare
-                rd[q][i] = fabs(d) > 0x1p-900 && fabs(d) < 0x1p900 ? 1.0 / d : 0.0;
+                rd[q][i] = mid_range(d) ? 1.0 / d : 0.0;  // kept where the correction step below holds
             }
         }
         __syncwarp(wmask);
@@ -275,7 +274,7 @@ __global__ void transient_fixed_kernel(TransientLaunch L) {
                 m &= m - 1;
                 acc = -b[k] * M[k * nt + i] + acc;
             }
-            if (!kTranExact) fin = fin && isfinite(acc);
+            if (!kTranExact) fin = fin && finite_bits(acc);
             b[i] = acc;
         }
         for (int i = nt - 1; i >= 0; --i) {
@@ -287,11 +286,19 @@ __global__ void transient_fixed_kernel(TransientLaunch L) {
                 m ^= 1u << k;
                 acc = -b[k] * M[k * nt + i] + acc;
             }
+            // acc / d as IEEE division gives it, by one step from the reciprocal where
+            // nothing leaves the normal range (and for +0; a -0 would lose its sign).
+            // With significands a, b in [1, 2) and u an ulp of a / b: r = (1 + e) / b,
+            // |e| <= b 2^-54, so acc r is less than u off, and where a / b is near the
+            // midpoint of two doubles the first product is one of the two, its remainder
+            // exact, and the corrected value at most |e| (u / 2 + t) off, t the distance
+            // to the midpoint.  t >= 2^-53 u / b is more than that, as b^2 < 4 - 2^-51.
             const double d = M[i * nt + i], r = rd[q][i];
             double x = acc * r;
-            x = fma(fma(-d, x, acc), r, x);  // the quotient to within its last bit
-            if (kTranExact || r == 0.0 || !isfinite(x)) x = acc / d;
-            if (!kTranExact) fin = fin && isfinite(x);
+            x = fma(fma(-d, x, acc), r, x);
+            const long long ab = __double_as_longlong(acc), rb = __double_as_longlong(r);
+            if (kTranExact || rb == 0 || !(ab == 0 || mid_range(acc))) x = acc / d;
+            if (!kTranExact) fin = fin && finite_bits(x);
             b[i] = x;
         }
     };
