@@ -22,7 +22,8 @@
 // addition of a zero product leaves the same bits; a probed unknown's quotient
 // is formed from all its parts, which gives its zeros their signs.  Values that
 // are not finite (whose product with a zero is not zero) and systems that
-// outgrow the slots go to the dense kernel.
+// outgrow the slots go to the dense kernel, as do sweeps of circuits whose
+// estimated fill (ac_plan.h) makes it the faster one.
 //
 // Bound: the FP64 pipe (64 cycles per warp instruction of an SM quarter) and,
 // with two warps per quarter, the chains between its instructions.  Op-amp,

@@ -12,6 +12,7 @@
 #include "transient_fixed.cuh"
 #include "ac.cuh"
 #include "ac_sparse.cuh"
+#include "ac_plan.h"
 #include "powergrid.cuh"
 
 using namespace sp;
@@ -463,44 +464,9 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
         gauss[k] = fine ? make_float4(mh, (float)(q.a - mh), sh, (float)(q.b - sh)) : make_float4(0.f, 0.f, NAN, 0.f);
     }
     const size_t bg = align256(sizeof(float4) * gauss.size());
-    // the AC matrix's real entries (ac_real_stamps' positions, in order of first
-    // touch) and the elements with imaginary ones; larger circuits have no AC sweep
-    std::vector<AcEntry> acent;
-    std::vector<AcReact> acreact;
-    int acvals = 0;
-    if (t->n <= kMaxDenseN) {
-        std::vector<char> seen((size_t)t->n * t->n, 0);
-        auto put = [&](int r, int col) {
-            if (r < 0 || col < 0 || seen[(size_t)col * t->n + r]) return;
-            seen[(size_t)col * t->n + r] = 1;
-            acent.push_back(AcEntry{(int16_t)r, (int16_t)col});
-        };
-        auto cond = [&](int i, int j) { put(i, i), put(j, j), put(i, j), put(j, i); };
-        auto vccs = [&](int op, int on, int cp, int cn) { put(op, cp), put(op, cn), put(on, cp), put(on, cn); };
-        for (int e = 0; e < c->num_elements; ++e) {
-            const sp_element& el = c->elements[e];
-            const int a0 = el.node[0], a1 = el.node[1], a2 = el.node[2], a3 = el.node[3], br = c->num_nodes + el.branch;
-            switch (el.kind) {
-                case SP_EL_R:
-                case SP_EL_D: cond(a0, a1); break;
-                case SP_EL_V:
-                case SP_EL_L: put(a0, br), put(br, a0), put(a1, br), put(br, a1); break;
-                case SP_EL_NMOS:
-                case SP_EL_PMOS: cond(a0, a2), vccs(a0, a2, a1, a2); break;
-                case SP_EL_NPN:
-                case SP_EL_PNP: cond(a1, a2), cond(a0, a2), vccs(a0, a2, a1, a2); break;
-                case SP_EL_BSIM3N:
-                case SP_EL_BSIM3P: cond(a0, a2), vccs(a0, a2, a1, a2), vccs(a0, a2, a3, a2); break;
-                default: break;
-            }
-            const bool b3 = el.kind == SP_EL_BSIM3N || el.kind == SP_EL_BSIM3P;
-            if (el.kind != SP_EL_C && el.kind != SP_EL_L && !b3) continue;
-            acreact.push_back(AcReact{el.kind, el.kind == SP_EL_L ? br : a0, a1, a2, a3, acvals});
-            acvals += b3 ? 5 : 1;
-        }
-        for (AcReact& r : acreact) r.val += (int)acent.size();
-    }
-    const size_t bae = align256(sizeof(AcEntry) * acent.size()), bar = align256(sizeof(AcReact) * acreact.size());
+    // the AC kernels' lists; larger circuits have no AC sweep
+    const AcLists ac = t->n <= kMaxDenseN ? ac_lists(t->n, c->num_nodes, c->elements, c->num_elements) : AcLists{};
+    const size_t bae = align256(sizeof(AcEntry) * ac.entries.size()), bar = align256(sizeof(AcReact) * ac.reacts.size());
     // every part in one buffer and one copy: a blocking copy costs several
     // microseconds whatever its size
     std::vector<char> stage;
@@ -520,8 +486,8 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     const size_t odrawn = part(bw, drawn.data(), sizeof(int) * drawn.size());
     const size_t otran = part(bt, tran.data(), sizeof(TransientEl) * tran.size());
     const size_t ogauss = part(bg, gauss.data(), sizeof(float4) * gauss.size());
-    const size_t oac = part(bae, acent.data(), sizeof(AcEntry) * acent.size());
-    part(bar, acreact.data(), sizeof(AcReact) * acreact.size());
+    const size_t oac = part(bae, ac.entries.data(), sizeof(AcEntry) * ac.entries.size());
+    part(bar, ac.reacts.data(), sizeof(AcReact) * ac.reacts.size());
     cudaError_t e = cudaMalloc(&t->dev, stage.size() + 256);
     if (e != cudaSuccess) {
         delete t;
@@ -543,9 +509,9 @@ int sp_topology_create(sp_ctx* ctx, const sp_circuit* c, sp_topology** out) {
     t->d_gauss32 = (const float4*)(b + ogauss);
     t->d_ac = b + oac;
     t->ac_react_off = bae;
-    t->num_ac_entries = (int)acent.size();
-    t->num_ac_reacts = (int)acreact.size();
-    t->num_ac_values = acvals;
+    t->num_ac_entries = (int)ac.entries.size();
+    t->num_ac_reacts = (int)ac.reacts.size();
+    t->num_ac_values = ac.values;
     t->d_drawn = (int*)(b + odrawn);
     t->num_drawn = (int)drawn.size();
     t->h_elements.assign(c->elements, c->elements + c->num_elements);
@@ -1615,6 +1581,52 @@ int sp_ac_frequencies(const sp_ac_config* cfg, double* freqs, int cap) {
     return (int)f.size();
 }
 
+// The sparse kernel's slots per lane (0: the dense kernel solves the sweep),
+// threads per block and resident warps per SM.
+struct AcSparsePlan {
+    int cap, block, warps;
+};
+
+// Warps per SM that `cap` slots leave resident, and the block of one to four warps that leaves the most.
+static int ac_sparse_warps(const sp_ctx* ctx, int n, int cap, int* block) {
+    int most = 0;
+    for (int w = 1; w <= 4; ++w) {
+        const size_t bytes = ac_sparse_warp_bytes(n, cap) * w;
+        if (bytes > (size_t)ctx->max_smem) break;
+        const int warps = std::min<int>((int)(228 * 1024 / (bytes + 1024)), 32) * w;
+        if (warps > most) *block = 32 * w, most = warps;
+    }
+    return most;
+}
+
+// Slots: the structural parts with as many again for fill where that leaves four
+// warps per SM, else the fill estimated plus one per unknown (samples of a warp
+// that pivot differently); then all that the same number of warps has room for.
+// A system that needs more is solved twice (again by the dense kernel), so an
+// estimate on the low side costs more than an idle slot.
+//
+// Sparse or dense: the time per unit is about ops (0.2 + 3.4 / warps) for the
+// sparse kernel (4.4 for a warp that has its SM to itself in a small sweep) and
+// ops max(0.55, 1.95 / warps) for the dense one, warps being those that an SM
+// holds and the sweep fills: fitted to 90 circuits of 5 to 28 unknowns.  4,096
+// samples x 41 frequencies, sparse / dense ms: 12 unknowns at 6 elements a node
+// 2.5 / 5.1, all tied to all 3.9 / 5.3; 14 at 6 8.5 / 7.4; 20 at 2 1.4 / 22, at 4
+// 10 / 22, at 10 44 / 23; 28 at 3 29 / 76, at 4 (outgrown) 133 / 77.
+static AcSparsePlan ac_sparse_plan(const sp_ctx* ctx, const sp_topology* t, int n, uint64_t units, int dense_warps) {
+    const int all = 2 * n * (n + 1) + n, need = std::min(all, t->ac_slots + n);
+    const int twice = std::min(all, 2 * (t->num_ac_entries + 4 * t->num_ac_reacts) + 4 * n);
+    AcSparsePlan p{std::max(need, twice), 32, 0};
+    p.warps = ac_sparse_warps(ctx, n, p.cap, &p.block);
+    if (p.warps < 4) p.warps = ac_sparse_warps(ctx, n, p.cap = need, &p.block);
+    if (!p.warps) return {0, 32, 0};
+    for (int block; p.cap < all && ac_sparse_warps(ctx, n, p.cap + 1, &block) == p.warps; p.block = block) ++p.cap;
+    const double fill = std::max(1.0, std::ceil((double)units / (32.0 * ctx->num_sms)));
+    const double sw = std::min(fill, (double)p.warps), dw = std::max(1.0, std::min(fill, (double)dense_warps / ctx->num_sms));
+    const double sparse = t->ac_ops * (0.2 + (fill > 1.0 ? 3.4 : 4.4) / sw), dense = t->ac_dense_ops * std::max(0.55, 1.95 / dw);
+    if (sparse > dense) return {0, 32, 0};
+    return p;
+}
+
 static int ac_locked(sp_ctx* ctx, sp_topology* t, const sp_newton_config* dc_cfg, const sp_ac_config* ac, uint64_t seed,
                      uint64_t first, uint64_t count, const double* d_table, uint32_t cols, double* d_probe,
                      uint8_t* d_status, cudaStream_t st) {
@@ -1685,23 +1697,19 @@ static int ac_locked(sp_ctx* ctx, sp_topology* t, const sp_newton_config* dc_cfg
         L.values = (double*)(base + bx + bp + bf + bs + bw);
         L.redo = redo;
         L.any_redo = redo + count;
-        // slots per thread: the structural parts with as many again for fill, the
-        // right-hand side and the pivots' reciprocals; at most every part there is.
-        // A system that needs more is solved by the dense kernel.
-        const int all = 2 * n * (n + 1) + n;
-        L.cap = std::min(all, 2 * (t->num_ac_entries + 4 * t->num_ac_reacts) + 4 * n);
-        while (L.cap > 1 && ac_sparse_warp_bytes(n, L.cap) > (size_t)ctx->max_smem) --L.cap;
-        // the block that leaves the most warps resident
-        int sblock = 32, most = 0;
-        for (int w = 1; w <= 4; ++w) {
-            const size_t bytes = ac_sparse_warp_bytes(n, L.cap) * w;
-            if (bytes > (size_t)ctx->max_smem) break;
-            const int warps = std::min<int>((int)(228 * 1024 / (bytes + 1024)), 32) * w;
-            if (warps > most) sblock = 32 * w, most = warps;
+        if (!t->ac_fill_known) {  // once per topology: a few microseconds to some tens
+            const sp_element* els = t->h_elements.data();
+            const AcFill f = ac_fill(n, t->num_nodes, els, t->num_elements, ac_lists(n, t->num_nodes, els, t->num_elements));
+            t->ac_slots = f.slots, t->ac_ops = (double)f.ops, t->ac_dense_ops = (double)f.dense_ops;
+            t->ac_fill_known = true;
         }
-        const uint64_t groups = (units + sblock - 1) / sblock;
-        const int sgrid = (int)std::min<uint64_t>(groups, (uint64_t)ctx->num_sms * std::max(1, most / (sblock / 32)));
-        SP_CUDA(ctx, launch_ac(L, grid, block, shared ? per * block : 0, sgrid, sblock, st), "AC launch");
+        const AcSparsePlan plan = ac_sparse_plan(ctx, t, n, units, grid * (block / 32));
+        L.cap = plan.cap;
+        const uint64_t groups = (units + plan.block - 1) / plan.block;
+        const int sgrid =
+            (int)std::min<uint64_t>(groups, (uint64_t)ctx->num_sms * std::max(1, plan.warps / (plan.block / 32)));
+        if (!plan.cap) SP_CUDA(ctx, cudaMemsetAsync(redo, 1, 4 * count + 4, st), "dense solves");
+        SP_CUDA(ctx, launch_ac(L, grid, block, shared ? per * block : 0, sgrid, plan.block, st), "AC launch");
     }
     return SP_OK;
 }

@@ -274,6 +274,9 @@ struct sp_topology {
     const void* d_ac = nullptr;  // AcEntry[num_ac_entries], then AcReact[num_ac_reacts] (inside `dev`)
     size_t ac_react_off = 0;     // bytes
     int num_ac_entries = 0, num_ac_reacts = 0, num_ac_values = 0;
+    bool ac_fill_known = false;  // ac_fill's estimate, made by the first FP64 AC sweep (under the context's lock)
+    int ac_slots = 0;
+    double ac_ops = 0.0, ac_dense_ops = 0.0;
     const float4* d_gauss32 = nullptr;  // [num_params] mean and sigma of Gaussian slots as FP32 pairs (inside `dev`)
     void* d_tran = nullptr;  // TransientEl[]: sources, capacitors, inductors, each in element order (inside `dev`)
     int* d_drawn = nullptr;  // slots whose kind is not SP_DRAW_FIXED, ascending (inside `dev`)

@@ -456,11 +456,13 @@ cudaError_t launch_lu_batch_cta(const double* mats, const double* rhs, int n, ui
 
 cudaError_t launch_ac(const AcLaunch& L, int grid, int block, size_t smem, int sparse_grid, int sparse_block,
                       cudaStream_t st) {
-    int vblock = 128;  // n^2 doubles of shared memory per sample
-    const size_t per = 8 * (size_t)L.c.n * L.c.n;
-    while (vblock > 32 && (per * vblock > 110 * 1024 || L.count / vblock < 304)) vblock >>= 1;
-    ac_values_kernel<<<(unsigned)((L.count + vblock - 1) / vblock), vblock, per * vblock, st>>>(L);
-    ac_sparse_kernel<<<sparse_grid, sparse_block, ac_sparse_warp_bytes(L.c.n, L.cap) * (sparse_block / 32), st>>>(L);
+    if (L.cap) {  // else every sample is marked for the dense kernel
+        int vblock = 128;  // n^2 doubles of shared memory per sample
+        const size_t per = 8 * (size_t)L.c.n * L.c.n;
+        while (vblock > 32 && (per * vblock > 110 * 1024 || L.count / vblock < 304)) vblock >>= 1;
+        ac_values_kernel<<<(unsigned)((L.count + vblock - 1) / vblock), vblock, per * vblock, st>>>(L);
+        ac_sparse_kernel<<<sparse_grid, sparse_block, ac_sparse_warp_bytes(L.c.n, L.cap) * (sparse_block / 32), st>>>(L);
+    }
     ac_kernel<<<grid, block, smem, st>>>(L);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
