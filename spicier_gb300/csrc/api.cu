@@ -793,7 +793,9 @@ static int newton_dc_locked(sp_ctx* ctx, const sp_topology* t, const sp_newton_c
         // 93.9 with no fallback launch at all (an empty miss list is the
         // common case; a long list gets 64 threads per SM)
         const int fblock = 32;
-        const int fgrid = std::max(1, std::min(ctx->num_sms * 2, (int)((count + fblock - 1) / fblock)));
+        // (blocks for lists of which each takes a sample, where teams of lanes do)
+        const uint64_t fper = L.fallback_team > 1 ? 1 : fblock;
+        const int fgrid = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)ctx->num_sms * 2, (count + fper - 1) / fper));
         const size_t fsmem = per * fblock;
         ProfScope prof(ctx, fname[prec], st);
         e = prec == SP_PREC_FP64_EXACT ? launch_newton_exact(L, true, fgrid, fblock, fsmem, st)

@@ -469,7 +469,8 @@ struct sink_int_tests<S, typename std::enable_if<S::kIntTests>::type> {
 };
 
 // Sinks that declare kTeam have `team` lanes (a power of two) that stamp the
-// same sample together, each evaluating its share of the BSIM3 devices.
+// same sample together, each evaluating its share of the BSIM3 devices; `lanes`
+// are those of the warp that stamp at the same time.
 template <class S, class = void>
 struct sink_team {
     static constexpr bool value = false;
@@ -495,12 +496,11 @@ __device__ inline Bsim3Out bsim3_eval_team(const DevCircuit& c, const DV& dv, si
         const double vs = el.node[2] >= 0 ? k.x(el.node[2]) : 0.0, vb = el.node[3] >= 0 ? k.x(el.node[3]) : 0.0;
         mine = bsim3_eval(el.kind == SP_EL_BSIM3P, [&](int i) { return dv(off + i, s); }, vg - vs, vd - vs, vb - vs);
     }
-    const unsigned lanes = (team == 32 ? 0xffffffffu : (1u << team) - 1u) << (threadIdx.x & 31 & -team);
     Bsim3Out r;
-    r.ids = __shfl_sync(lanes, mine.ids, turn, team);
-    r.gds = __shfl_sync(lanes, mine.gds, turn, team);
-    r.gm = __shfl_sync(lanes, mine.gm, turn, team);
-    r.gmbs = __shfl_sync(lanes, mine.gmbs, turn, team);
+    r.ids = __shfl_sync(k.lanes, mine.ids, turn, team);
+    r.gds = __shfl_sync(k.lanes, mine.gds, turn, team);
+    r.gm = __shfl_sync(k.lanes, mine.gm, turn, team);
+    r.gmbs = __shfl_sync(k.lanes, mine.gmbs, turn, team);
     return r;
 }
 #endif

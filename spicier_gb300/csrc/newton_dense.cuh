@@ -109,17 +109,19 @@ struct MixedSinkRec : MixedSink {
     }
 };
 
-// A sink, or (TEAM) the same for a sample that `team` lanes hold.
+// A sink, or (TEAM) the same for a sample that `team` lanes hold; lanes: those
+// that stamp together, one team where teams go their own ways or the whole warp.
 template <class S>
 struct TeamSink : S {
     static constexpr bool kTeam = true;
     int team;
+    unsigned lanes;
     template <class... A>
-    __device__ TeamSink(int t, A... a) : S{a...}, team(t) {}
+    __device__ TeamSink(int t, unsigned l, A... a) : S{a...}, team(t), lanes(l) {}
 };
 template <bool TEAM, class S, class... A>
-__device__ inline auto make_sink(int team, A... a) {
-    if constexpr (TEAM) return TeamSink<S>(team, a...);
+__device__ inline auto make_sink(int team, unsigned lanes, A... a) {
+    if constexpr (TEAM) return TeamSink<S>(team, lanes, a...);
     else return S{a...};
 }
 
@@ -452,7 +454,7 @@ __device__ inline int newton_run(const DevCircuit& c, const DV& dv, size_t s,
         if (PREC == SP_PREC_FP64) {
             for (int i = 0; i < n * n; ++i) w.A[i] = 0.0;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            auto k = make_sink<TEAM, PlainSink>(w.team, w.A, w.v, w.x, n);
+            auto k = make_sink<TEAM, PlainSink>(w.team, team_lanes(w.team), w.A, w.v, w.x, n);
             stamp_all(c, dv, s, k, mode, aux);
             if (!lu_solve_fp64(n, w.A, w.v)) {
                 iters = it + 1;
@@ -471,7 +473,7 @@ __device__ inline int newton_run(const DevCircuit& c, const DV& dv, size_t s,
         } else {
             for (int i = 0; i < n * n; ++i) w.J[i] = 0.0f;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            auto k = make_sink<TEAM, MixedSink>(w.team, w.J, w.v, w.x, n);
+            auto k = make_sink<TEAM, MixedSink>(w.team, team_lanes(w.team), w.J, w.v, w.x, n);
             stamp_all(c, dv, s, k, mode, aux);
             for (int i = 0; i < n; ++i) w.d[i] = (float)(-w.v[i]);
             if (!lu_solve_fp32(n, w.J, w.d)) {
@@ -522,14 +524,14 @@ __device__ inline int newton_run_warp(const DevCircuit& c, const SoA& dv, size_t
         if (PREC == SP_PREC_FP64) {
             for (int i = 0; i < n * n; ++i) w.A[i] = 0.0;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            auto k = make_sink<TEAM, PlainSinkRec>(w.team, w.A, w.v, w.x, n, lane);
+            auto k = make_sink<TEAM, PlainSinkRec>(w.team, 0xffffffffu, w.A, w.v, w.x, n, lane);
             stamp_all(c, dv, s, k, STAMP_PLAIN, 0.0);
             __syncwarp();
             ok = lu_solve_warp<double>(n, lane, w.A, w.v, k.rows, plain);
         } else {
             for (int i = 0; i < n * n; ++i) w.J[i] = 0.0f;
             for (int i = 0; i < n; ++i) w.v[i] = 0.0;
-            auto k = make_sink<TEAM, MixedSinkRec>(w.team, w.J, w.v, w.x, n, lane);
+            auto k = make_sink<TEAM, MixedSinkRec>(w.team, 0xffffffffu, w.J, w.v, w.x, n, lane);
             stamp_all(c, dv, s, k, STAMP_PLAIN, 0.0);
             __syncwarp();
             for (int i = 0; i < n; ++i) w.d[i] = (float)(-w.v[i]);
@@ -560,7 +562,7 @@ __device__ inline int newton_run_warp(const DevCircuit& c, const SoA& dv, size_t
 template <bool TEAM = false, class DV>
 __device__ inline double kcl_residual(const DevCircuit& c, const DV& dv, size_t s, Work& w) {
     for (int i = 0; i < c.n; ++i) w.v[i] = 0.0;
-    auto k = make_sink<TEAM, ResidSink>(w.team, w.v, w.x);
+    auto k = make_sink<TEAM, ResidSink>(w.team, team_lanes(w.team), w.v, w.x);
     stamp_all(c, dv, s, k, STAMP_PLAIN, 0.0);
     double r = 0.0;
     for (int i = 0; i < c.num_nodes; ++i) r = fmax(r, fabs(w.v[i]));
@@ -668,9 +670,9 @@ __global__ void newton_primary_kernel(NewtonLaunch L) {
     load_start(L, sd, w, warm);
     code = newton_run_warp<PREC, TEAM>(L.c, L.dv, sd, L.cfg, w, it, active, &plain);
     if (!active) return;
-    if (!plain) {
+    if (!plain) {  // by single lanes: the teams of a warp part here
         load_start(L, s, w, warm);
-        code = newton_run<PREC, TEAM>(L.c, L.dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
+        code = newton_run<PREC>(L.c, L.dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
     }
 #endif
     const bool lead = !TEAM || (threadIdx.x & (L.team - 1)) == 0;  // the others hold the same values
@@ -772,69 +774,80 @@ __device__ inline int source_stepping(const NewtonLaunch& L, const DV& dv, size_
 
 namespace SP_KERNEL_NS {
 
+// The fallback chain of one sample, held by `team` lanes.  All of them take the
+// same branches: what decides one comes from values that each has computed
+// alike, or from the sample's row, which changes only in put_row.
+template <int PREC, bool TEAM, class DV>
+__device__ inline void fallback_sample(const NewtonLaunch& L, const DV& dv, size_t s, Work& w, unsigned team) {
+    const int n = L.c.n;
+    const bool warm = L.x0 != nullptr || L.lin != nullptr;  // listed samples started warm
+    const bool lead = team_leads<TEAM>(team);
+    w.team = (int)team;
+    if (L.redraw.derived) redraw_sample(L.c, L.redraw, L.dv.stride, s);
+    int total = L.iters ? L.iters[s] : 0;
+    uint8_t flags = warm ? SP_ST_FLAG_WARM : 0;
+    // A stage succeeds only if it converged with a finite iterate (the
+    // reference's convergence test passes NaN iterates).
+    auto ok = [&](int code) {
+        if (code != NR_CONVERGED) return false;
+        for (int i = 0; i < n; ++i)
+            if (!isfinite(L.x[s * n + i])) return false;
+        return true;
+    };
+    int code = NR_MAXITER;
+    // the specialised kernel has already restarted this sample cold (status
+    // flag), so the chain continues with gmin stepping
+    const bool cold_done = warm && L.status && (L.status[s] & SP_ST_FLAG_COLD);
+    team_sync<TEAM>(team);  // read before the leader writes them
+    if (cold_done) flags |= SP_ST_FLAG_COLD;
+    if (warm && !cold_done) {
+        flags |= SP_ST_FLAG_COLD;
+        load_start(L, s, w, false);
+        int it = 0;
+        code = newton_run<PREC, TEAM>(L.c, dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
+        total += it;
+        put_row<TEAM>(team, n, L.x + s * n, [&](int i) { return w.x[i]; });
+    }
+    if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_GMIN)) {
+        flags |= SP_ST_FLAG_GMIN;
+        code = gmin_stepping<PREC, TEAM>(L, dv, s, w, total);
+    }
+    if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_SOURCE)) {
+        flags |= SP_ST_FLAG_SOURCE;
+        code = source_stepping<PREC, TEAM>(L, dv, s, w, total);
+    }
+    for (int i = 0; i < n; ++i) w.x[i] = L.x[s * n + i];
+    uint8_t st = finish_status(code, w, n) | flags;
+    const double res = L.resid ? kcl_residual<TEAM>(L.c, dv, s, w) : 0.0;
+    if (lead && L.iters) L.iters[s] = total;
+    if (lead && L.status) L.status[s] = st;
+    if (lead && L.resid) L.resid[s] = res;
+}
+
 // Phase 2: the fallback chain for the samples phase 1 missed (grid-stride
-// over the miss list, whose length is only known on the device).
+// over the miss list, whose length is only known on the device; one-warp blocks).
 template <int PREC, bool TEAM = false>
 __global__ void newton_fallback_kernel(NewtonLaunch L) {
     extern __shared__ __align__(16) unsigned char smem[];
     pdl_wait();
     pdl_trigger();
     Work w = make_work<PREC>(smem, L.c.n, blockDim.x, threadIdx.x);
-    const int n = L.c.n;
-    const bool warm = L.x0 != nullptr || L.lin != nullptr;  // listed samples started warm
     const unsigned int misses = *L.fail_count;
     const SoACg dv{L.dv.p, L.dv.stride};
-    // A short list leaves most lanes idle: each sample then has a team of lanes,
-    // every one of them with its data.  All of them take the same branches: what
-    // decides one comes from values that each has computed alike, or from the
-    // sample's row, which changes only in put_row.
-    const unsigned team = TEAM && (uint64_t)misses * L.fallback_team <= (uint64_t)gridDim.x * blockDim.x ? L.fallback_team : 1;
-    const bool lead = team_leads<TEAM>(team);
-    w.team = (int)team;
+    // A list of at most a sample per block: a team of the block's lanes takes it,
+    // every one of them with its data.  Longer lists go to single lanes: teams of
+    // one warp part at the first stage of different length, and every shuffle and
+    // barrier of theirs then runs once per team (608 chains of eight devices, all
+    // failing: 447 ms with several teams in a warp, or teams of one lane; 112 so).
+    if (TEAM && misses <= gridDim.x) {
+        if (blockIdx.x < misses && threadIdx.x < (unsigned)L.fallback_team)
+            fallback_sample<PREC, true>(L, dv, L.fail_list[blockIdx.x], w, (unsigned)L.fallback_team);
+        return;
+    }
     // neighbours in the list go to different blocks: chains differ in length at
     // every level, and lanes of one warp wait for each other there
-    for (unsigned int j = threadIdx.x / team * gridDim.x + blockIdx.x; j < misses; j += gridDim.x * (blockDim.x / team)) {
-        const size_t s = L.fail_list[j];
-        if (L.redraw.derived) redraw_sample(L.c, L.redraw, L.dv.stride, s);
-        int total = L.iters ? L.iters[s] : 0;
-        uint8_t flags = warm ? SP_ST_FLAG_WARM : 0;
-        // A stage succeeds only if it converged with a finite iterate (the
-        // reference's convergence test passes NaN iterates).
-        auto ok = [&](int code) {
-            if (code != NR_CONVERGED) return false;
-            for (int i = 0; i < n; ++i)
-                if (!isfinite(L.x[s * n + i])) return false;
-            return true;
-        };
-        int code = NR_MAXITER;
-        // the specialised kernel has already restarted this sample cold (status
-        // flag), so the chain continues with gmin stepping
-        const bool cold_done = warm && L.status && (L.status[s] & SP_ST_FLAG_COLD);
-        team_sync<TEAM>(team);  // read before the leader writes them
-        if (cold_done) flags |= SP_ST_FLAG_COLD;
-        if (warm && !cold_done) {
-            flags |= SP_ST_FLAG_COLD;
-            load_start(L, s, w, false);
-            int it = 0;
-            code = newton_run<PREC, TEAM>(L.c, dv, s, L.cfg, STAMP_PLAIN, 0.0, w, it);
-            total += it;
-            put_row<TEAM>(team, n, L.x + s * n, [&](int i) { return w.x[i]; });
-        }
-        if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_GMIN)) {
-            flags |= SP_ST_FLAG_GMIN;
-            code = gmin_stepping<PREC, TEAM>(L, dv, s, w, total);
-        }
-        if (!ok(code) && (L.cfg.fallback & SP_FALLBACK_SOURCE)) {
-            flags |= SP_ST_FLAG_SOURCE;
-            code = source_stepping<PREC, TEAM>(L, dv, s, w, total);
-        }
-        for (int i = 0; i < n; ++i) w.x[i] = L.x[s * n + i];
-        uint8_t st = finish_status(code, w, n) | flags;
-        const double res = L.resid ? kcl_residual<TEAM>(L.c, dv, s, w) : 0.0;
-        if (lead && L.iters) L.iters[s] = total;
-        if (lead && L.status) L.status[s] = st;
-        if (lead && L.resid) L.resid[s] = res;
-    }
+    for (unsigned int j = threadIdx.x * gridDim.x + blockIdx.x; j < misses; j += gridDim.x * blockDim.x)
+        fallback_sample<PREC, false>(L, dv, L.fail_list[j], w, 1);
 }
 
 }  // namespace SP_KERNEL_NS
