@@ -833,7 +833,7 @@ __global__ void newton_fallback_kernel(NewtonLaunch L) {
     pdl_trigger();
     Work w = make_work<PREC>(smem, L.c.n, blockDim.x, threadIdx.x);
     const unsigned int misses = *L.fail_count;
-    const SoACg dv{L.dv.p, L.dv.stride};
+    const SoAOwn dv{L.dv.p, L.dv.stride};
     // A list of at most a sample per block: a team of the block's lanes takes it,
     // every one of them with its data.  Longer lists go to single lanes: teams of
     // one warp part at the first stage of different length, and every shuffle and
