@@ -736,16 +736,20 @@ static int newton_dc_locked(sp_ctx* ctx, const sp_topology* t, const sp_newton_c
                                         : work_bytes_per_thread<SP_PREC_FP64>(t->n);
     // The BSIM3 devices of a sample go to the lanes of a team: an evaluation is
     // about 350 FP64 instructions of 64 cycles each, however few lanes take part.
-    // In the primary kernel that pays while single lanes would leave quarters of
-    // SMs without a warp (three devices: 2,000 samples 5.7 -> 4.6 ms, 8,192
-    // 6.6 -> 6.1, but 12,000 6.4 -> 7.8, a call with its fallback); the fallback
-    // decides by the length of its list (8,192 samples, 169 of them listed: 6.7
-    // -> 3.4 ms).
+    // In the primary kernel that pays up to two warps per quarter of an SM, which
+    // keep its FP64 pipe busy (a dependent instruction takes about 130 cycles):
+    // primary with single lanes / teams, ms at 4, 8 and 8.5 warps' worth of lanes
+    // per SM, three devices 2.22 / 1.24, 2.23 / 1.71, 2.41 / 3.79 (mixed), 2.26 /
+    // 1.50, 2.27 / 2.10, 2.46 / 2.10 (FP64); two devices 1.79 / 1.27, 1.90 / 1.87,
+    // 2.38 / 4.16 (mixed); eight 6.6 / 2.3, 6.6 / 3.1, 7.0 / 5.9.  With more
+    // devices than lanes the last round idles: eleven in FP64 9.3 / 7.9 at 6, 9.2 /
+    // 11.4 at 7.  The fallback decides by the length of its list.
     int team = 1;
     while (team < 8 && team < t->dc.num_b3) team *= 2;
     if (prec == SP_PREC_FP64_EXACT) team = 1;  // (no instances of those kernels)
     L.fallback_team = team;
-    if (!use_spec && count * team <= (uint64_t)ctx->num_sms * 32 * 7) L.team = team;
+    const uint64_t team_warps = kprec == SP_PREC_FP64 && t->dc.num_b3 > team ? 6 : 8;
+    if (!use_spec && count * team <= (uint64_t)ctx->num_sms * 32 * team_warps) L.team = team;
     const uint64_t lanes = count * L.team;
     int block = pick_block(per, ctx->max_smem, lanes, ctx->num_sms);
     if (!block) return fail(ctx, SP_ERR_INVALID_DIMENSION, "MNA size %d does not fit shared memory", t->n);
