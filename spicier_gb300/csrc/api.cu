@@ -1280,8 +1280,8 @@ static int grid_validate(sp_ctx* ctx, const sp_grid_config* c, uint64_t count) {
     if (count > 0x7fffffffull)
         return fail(ctx, SP_ERR_BATCH_TOO_LARGE, "Batch size %llu exceeds maximum %llu", (unsigned long long)count,
                     0x7fffffffull);
-    const size_t smem = grid_smem_bytes(*c, c->precision == SP_PREC_MIXED ? 4 : 8);
-    if (smem > (size_t)ctx->max_smem) return fail(ctx, SP_ERR_INVALID_DIMENSION, "grid too large for shared memory");
+    if (grid_launch_smem(*c, ctx->max_smem) > (size_t)ctx->max_smem)
+        return fail(ctx, SP_ERR_INVALID_DIMENSION, "grid too large for shared memory");
     return SP_OK;
 }
 

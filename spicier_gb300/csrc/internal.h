@@ -65,6 +65,8 @@ cudaError_t launch_transient_fast(const TransientLaunch& L, int block, size_t sm
 struct LadderLaunch;
 struct GridLaunch;
 cudaError_t launch_grid(const GridLaunch& L, int precision, cudaStream_t st);
+// Dynamic shared memory of that launch.
+size_t grid_launch_smem(const sp_grid_config& c, int max_smem);
 // Ladder transient launchers (ladder.cuh): one block of `threads` per instance.
 cudaError_t launch_ladder_exact(const LadderLaunch& L, int grid, int threads, size_t smem, cudaStream_t st);
 cudaError_t launch_ladder_fast(const LadderLaunch& L, int precision, int grid, int threads, size_t smem,

@@ -567,6 +567,11 @@ cudaError_t launch_yield(const double* v, uint64_t rows, uint32_t ld, const uint
     return cudaGetLastError();
 }
 
+size_t grid_launch_smem(const sp_grid_config& c, int max_smem) {
+    return c.precision == SP_PREC_MIXED ? grid_mixed_smem(c.rows * c.cols + 1, c.restart, max_smem).total
+                                        : grid_smem_bytes(c, 8);
+}
+
 cudaError_t launch_grid(const GridLaunch& L, int precision, cudaStream_t st) {
     if (precision == SP_PREC_MIXED) {
         const int n = L.cfg.rows * L.cfg.cols + 1, nq = grid_mixed_rows(n);
