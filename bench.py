@@ -772,7 +772,7 @@ def main():
                              "roofline": {"bound": "fp64", "achieved": a, "peak": fp64_peak, "unit": "TFLOP/s",
                                           "frac": a / fp64_peak, "flops": fl,
                                           "per_unit": "45 FP64 flops per ladder node per Newton iteration",
-                                          "note": "latency of the serial step chain (a warp per ladder) binds, "
+                                          "note": "latency of the serial step chain (a CTA per ladder) binds, "
                                                   "not the pipe"}}
         sample3 = 64
         with oracle.math_mode("cr"):

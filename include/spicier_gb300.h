@@ -573,6 +573,8 @@ typedef struct sp_ac_config {
     int32_t probe[8];
     int32_t precision;   /* SP_PREC_FP64: the reference's FP64 LU order;       */
                          /* SP_PREC_MIXED: FP32 complex LU + FP64 refinement  */
+                         /* (a dense solve: slower than FP64, which works on  */
+                         /* the circuit's pattern; op-amp 0.42 times as fast) */
     int32_t refine;      /* mixed: residual refinement steps (0 -> 3)          */
 } sp_ac_config;
 

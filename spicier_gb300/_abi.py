@@ -207,7 +207,8 @@ def ac_config(fstart: float, fstop: float, num_points: int, sweep: int = SP_AC_D
     """AC sweep settings (AcParams, ac.rs:30-40): frequency range and points (total for SP_AC_LIN, per decade or
     octave otherwise), the recorded unknowns (1..8), the stimulus (-1: every V source at AC magnitude 1, as
     the reference's ac_info default; else the element index of the one source), and the precision
-    (SP_PREC_FP64: the reference's LU order; SP_PREC_MIXED: FP32 LU with `refine` FP64 refinement steps)."""
+    (SP_PREC_FP64: the reference's LU order, on the circuit's pattern; SP_PREC_MIXED: dense FP32 LU with `refine`
+    FP64 refinement steps, the slower one)."""
     c = SpAcConfig()
     c.fstart, c.fstop, c.num_points, c.sweep, c.source = fstart, fstop, num_points, sweep, source
     c.precision, c.refine = precision, refine

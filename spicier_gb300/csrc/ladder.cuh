@@ -13,8 +13,8 @@
 // What bounds it: the FP64 pipe (two lanes per clock and SM, about 20 FP64
 // operations per section and Newton iteration) once several ladders share an
 // SM, and the serial chain of the longest ladder when few do.  A ladder's
-// arrays therefore live in shared memory (about 80 bytes a section, five
-// ladders of 512 sections per SM), the per-section work is spread over the
+// arrays therefore live in shared memory (about 90 bytes a section, four
+// ladders of 512 sections per SM; FP64 120 bytes, three), the per-section work is spread over the
 // CTA, and the chain inside an iteration is kept to the elimination's
 // dependent divisions.  One warp per ladder with its arrays in L2, the
 // partition's 64-bit index divisions, a branch per division and bank conflicts

@@ -283,8 +283,8 @@ __device__ __forceinline__ unsigned abs_bits(float x) { return __float_as_uint(x
 // on it: the pivot search compares bit patterns, the substitution's quotients
 // come from the pivots' reciprocals, and pivots of +-1 (voltage-source rows)
 // divide nothing.  The op-amp's 12 x 12 matrix takes about 100 of the dense
-// 780 updates; its 65,536-sample FP64 sweep went from 1,447 to 636 us, the
-// 1,024-sample 5-unknown amplifier's from 85 to 70.
+// 780 updates; its 65,536-sample FP64 sweep went from 1,447 to 583 us, the
+// 1,024-sample 5-unknown amplifier's from 85 to 66.
 template <class T>
 __device__ inline bool lu_solve_warp(int n, int lane, Il<T> A, Il<T> b, unsigned rows, bool* plain) {
     bool ok = true, fin = true;

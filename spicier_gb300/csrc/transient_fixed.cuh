@@ -21,7 +21,8 @@
 // are kept), the substitution's divisions (reciprocals of the diagonal are
 // kept, with one correction step) and, outside the exact unit, the factor's
 // zeros.  16,384 samples of a 9-unknown RLC network, 150 trapezoidal steps:
-// 6.2 -> 1.5 ms.
+// 6.2 -> 1.5 ms (TR-BDF2 holds two factors a sample; runs of one or two steps lose a
+// little: 16,384 samples of 10 unknowns, 2 steps, 0.42 ms instead of 0.36).
 #pragma once
 #include <math_constants.h>
 
